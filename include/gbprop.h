@@ -263,7 +263,7 @@ gbprop_status gbprop_autotune(gbprop_handle h, int* variant);
  * row l in the B-spline overlap metric) -- the analysis of the reference's hydrogen example
  * (examples/tensor/helium_stabilization_sae/analysis.py:92-160, a dense generalized
  * eigensolver per l there).  Here: inertia counts of banded LDL^T factorisations of
- * H - sigma S, bisection to the double-precision eigenvalue (one GPU thread per state) and
+ * H - sigma S, bisection to the double-precision eigenvalue (one GPU CTA per state) and
  * inverse iteration for the vector, normalised in the S metric (sign arbitrary).
  *   h_bands  DEVICE, nrows x (2kd+1) x nr doubles: h_bands[(l (2kd+1) + d) nr + i] = H_l(i, i+d-kd)
  *            (symmetric; the lower half and the diagonal are read)
