@@ -126,9 +126,12 @@ struct gbprop_ctx {
     long long arnoldi_launches = 0;
     long long graph_launches = 0;
     int band_variant = 1;             // tile shape of the band kernel (autotuner)
-    int expm_max_cluster = 16;        // 1 when the handle is advanced inside a batch
+    int expm_max_cluster = 16;        // 1 inside a large batch
+    bool in_batch = false;
     bool inv_ok = false;              // solves run through the banded approximate inverse
-    InvTab inv[2] = {};               // [0]: U^-1, [1]: U^-T
+    InvTab inv[2] = {};               // the Krylov-precision solves: [0]: U^-1, [1]: U^-T
+    InvTab sinv[2] = {};              // the FP64-accurate solves of the state (same tables, own chunking)
+    InvTab pinv[2] = {};              // those in place: one chunk where that is as fast as a copy
 
     ~gbprop_ctx() {
         if (graph) cudaGraphExecDestroy(graph);
@@ -266,6 +269,8 @@ struct HostInvTab {
     double contraction = 0.0;          // simulated error ratio of one refinement pass
     std::vector<float> m;              // (w+1) x npad
     std::vector<double> u;             // (kd+1) x npad
+    int ks = 0;
+    std::vector<unsigned short> mf;    // m in bfloat16 parts in the order of the matrix instruction's fragments (InvTab)
 };
 
 // U~ = U (dir 0) or U^T in reversed coordinates q = n-1-p (dir 1): upper triangular in q.
@@ -315,6 +320,24 @@ HostInvTab build_inv_tab(const std::vector<double>& U, int n, int kd, int dir) {
     t.m.assign((size_t)(w + 1) * t.npad, 0.0f);
     for (int j = 0; j <= w; ++j)
         for (int q = 0; q + j < n; ++q) t.m[(size_t)j * t.npad + q] = (float)inv[(size_t)j * n + q];
+    t.ks = ((w + 16 + 15) / 16 + kSolveFrags - 1) / kSolveFrags * kSolveFrags;
+    t.mf.assign((size_t)((n + 15) / 16) * t.ks * 3 * 256, 0);
+    for (int j = 0; j <= w; ++j)
+        for (int q = 0; q + j < n; ++q) {
+            const int r = q % 16, c = r + j;
+            const size_t lane = (size_t)(r % 8) * 4 + c % 8 / 2, e = c % 2 + 2 * (r >= 8) + 4 * (c % 16 >= 8);
+            const size_t at = (((size_t)(q / 16) * t.ks + c / 16) * 3 * 32 + lane) * 8 + e;
+            float v = t.m[(size_t)j * t.npad + q];
+            for (int part = 0; part < 3; ++part) {
+                uint32_t bits;
+                std::memcpy(&bits, &v, 4);
+                bits &= 0xffff0000u;
+                float h;
+                std::memcpy(&h, &bits, 4);
+                t.mf[at + (size_t)part * 256] = (unsigned short)(bits >> 16);
+                v -= h;
+            }
+        }
     t.u.assign((size_t)(kd + 1) * t.npad, 0.0);
     for (int d = 0; d <= kd; ++d)
         for (int q = 0; q + d < n; ++q) t.u[(size_t)d * t.npad + q] = ut(q, q + d);
@@ -371,6 +394,9 @@ HostInvTab build_inv_tab(const std::vector<double>& U, int n, int kd, int dir) {
         }
         prev = e;
     }
+    // the device's products are split ones on units that truncate where this simulation rounds: room
+    // for an eight times weaker pass
+    while (t.ok && t.refine < kMaxRefine && std::pow(8.0 * t.contraction, t.refine + 1) > 1e-15) ++t.refine;
     return t;
 }
 
@@ -535,83 +561,109 @@ SchedEntry sched_entry(const double* vals, int nf, double dt_re, double dt_im) {
     return e;
 }
 
-// Chunking of the inverse solve.  `wide` spreads one problem's rows over the GPU: the
-// chunk count minimises (waves of CTAs) x (FP64 residual elements of one CTA, halo
-// included), the refinement being FP64-issue-bound; otherwise (batches, where other
-// problems fill the GPU) the fewest chunks are used.  The chunk's slices of M and U~ are
-// staged in shared memory when one CTA's share stays within 220 KB, else read through L2.
-void set_inv_chunks(gbprop_ctx* h, bool wide) {
-    const int n = h->nr, kd = h->kd, sms = grid_reduce_blocks();
-    for (int dir = 0; dir < 2; ++dir) {
-        InvTab& t = h->inv[dir];
-        const int P = t.refine, w = t.w;
-        auto chunk_of = [&](int nch) { return std::max(4, ((n + nch - 1) / nch + 3) & ~3); };
-        // the table serves the FP64-accurate solve and, on mixed handles, the complex64 basis
-        // solve (which also stages the FP32 pairs of U~): both must fit
-        const bool mixed = h->prec != GBPROP_FP64;
-        auto smem_of = [&](int chunk, int stage) {
-            size_t mx = 0;
-            for (int q0 = 0; q0 < n; q0 += chunk) {
-                mx = std::max(mx, inv_smem_bytes(n, q0, chunk, P, w, kd, stage, 1));
-                if (mixed) mx = std::max(mx, inv_smem_bytes_mixed(n, q0, chunk, w, kd, stage));
-            }
-            return mx;
-        };
-        // cost ~ (waves of resident CTAs) x (elements one CTA processes over all passes); CTAs
-        // that fit two per SM count as half a wave each (their latency-bound phases overlap)
-        auto cost = [&](int chunk, int stage) {
-            const int nch = (n + chunk - 1) / chunk;
-            long work = 0;
-            for (int k = 0; k <= P; ++k) work += std::min(n, chunk + (P - k) * (w + kd) + w);
-            const size_t sm = smem_of(chunk, stage) + 1024;
-            const int per_sm = std::max(1, std::min(2, (int)((size_t)228 * 1024 / sm)));
-            const long waves = ((long)h->nl * nch + (long)sms * per_sm - 1) / ((long)sms * per_sm);
-            return waves * work * 2 / per_sm;
-        };
-        int best = -1, best_stage = 0;
-        long best_cost = 0;
-        for (int stage = 1; stage >= 0 && best < 0; --stage) {
-            for (int nch = 1; nch <= 16; ++nch) {
-                const int chunk = chunk_of(nch);
-                if (nch > 1 && chunk < 32) break;
-                if (smem_of(chunk, stage) > (size_t)220 * 1024) continue;
-                const long c = cost(chunk, stage);
-                if (best < 0 || (wide ? c < best_cost : false)) {
-                    best = chunk;
-                    best_cost = c;
-                    best_stage = stage;
-                }
-                if (!wide && best >= 0) break;
-            }
-        }
-        if (best < 0) { best = chunk_of(1); best_stage = 0; }
-        t.chunk = best;
-        t.nchunks = (n + best - 1) / best;
-        t.stage = best_stage;
+// Shape of the inverse solve (k_solve_rows): rows per CTA and radial chunk.  SM cycles of one CTA,
+// from its instruction counts (four issue slots a cycle; an FP64 warp instruction holds the SM's
+// FP64 unit for 16 cycles) plus the latency of the barrier-separated phases:
+//   band product   one tile (16 outputs x 8 planes) per warp at a time, about 80 cycles a k step
+//   FP32 residual  about 190 instructions and, for an FP64 right-hand side, 2 FP64 ones per 32
+//                  complex elements
+//   FP64 residual  2 (kd+1) FP64 instructions per 32 complex elements
+//   FP64 update    2 to 6 FP64 instructions per 32 complex elements
+constexpr size_t kSolveSmem = (size_t)200 * 1024;
+constexpr int kSolveFixedCycles = 4000;
+
+double solve_cta_cycles(const InvTab& t, int chunk, int rg, int r64, int warps) {
+    const int P = r64 ? t.refine : 1, hop = t.w + t.kd, cl = std::min(chunk, t.n);
+    double c = 0.0;
+    for (int k = 0; k <= P; ++k) {
+        const int Rk = std::min(t.n, cl + (P - k) * hop), Rr = std::min(t.n, Rk + t.w);
+        const int tiles = (Rk + 15) / 16 * ((2 * rg + 7) / 8);
+        c += (double)((tiles + warps - 1) / warps) * t.ks * 80;
+        if (r64 && k > 0) c += rg * Rk / 32.0 * (k == P ? 6 : 2) * 16;
+        if (k == 0) continue;
+        if (k == 1 && (P >= 2 || !r64)) c += rg * Rr / 32.0 * (190 / 4 + (r64 ? 32 : 0));
+        else c += rg * Rr / 32.0 * 2 * (t.kd + 1) * 16;
     }
+    return c;
 }
 
-// Use `nch` radial chunks for the solves of direction `dir`, staging the slices when they fit;
-// false if one CTA's share exceeds the shared-memory budget either way.
-bool set_inv_chunk_count(gbprop_ctx* h, int dir, int nch) {
-    InvTab& t = h->inv[dir];
-    const int n = h->nr, kd = h->kd, P = t.refine, w = t.w;
-    const bool mixed = h->prec != GBPROP_FP64;
-    const int chunk = std::max(4, ((n + nch - 1) / nch + 3) & ~3);
-    for (int stage = 1; stage >= 0; --stage) {
-        size_t mx = 0;
-        for (int q0 = 0; q0 < n; q0 += chunk) {
-            mx = std::max(mx, inv_smem_bytes(n, q0, chunk, P, w, kd, stage, 1));
-            if (mixed) mx = std::max(mx, inv_smem_bytes_mixed(n, q0, chunk, w, kd, stage));
-        }
-        if (mx <= (size_t)220 * 1024) {
+int log2_of(int rg) { return rg >= 16 ? 4 : rg >= 8 ? 3 : rg >= 4 ? 2 : rg >= 2 ? 1 : 0; }
+
+size_t solve_smem(InvTab t, int chunk, int rg, int stage, int r64) {
+    t.chunk = chunk;
+    t.lg = log2_of(rg);
+    t.stage = stage;
+    inv_shape(t, r64);
+    return t.ly.bytes;
+}
+
+int chunk_of(int n, int nch) { return ((n + nch - 1) / nch + 15) & ~15; }
+
+// Use chunks of `chunk` elements and 2^lg rows; false if they do not fit in shared memory.
+bool set_solve_shape(InvTab& t, int chunk, int lg, int r64) {
+    for (int st = 1; st >= 0; --st)
+        if (solve_smem(t, chunk, 1 << lg, st, r64) <= kSolveSmem) {
+            t.lg = lg;
             t.chunk = chunk;
-            t.nchunks = (n + chunk - 1) / chunk;
-            t.stage = stage;
+            t.nchunks = (t.n + chunk - 1) / chunk;
+            t.stage = st;
+            inv_shape(t, r64);
             return true;
         }
-    }
     return false;
+}
+
+// Modelled time of that shape, alone on the GPU: SM cycles of the busiest SM, the fixed part shared by
+// up to two resident CTAs.  In a batch: SM cycles of all CTAs (the other problems fill what is free) and,
+// with the weight of the best of 0, 8 and 32 on batches of 4 to 24 problems, those of one, which the
+// problem's chain of kernels waits for.
+double solve_cost(const gbprop_ctx* h, const InvTab& t, int chunk, int lg, int r64, int batch) {
+    const int sms = grid_reduce_blocks();
+    const long ctas = (long)((h->nl + (1 << lg) - 1) >> lg) * ((t.n + chunk - 1) / chunk);
+    const double one = solve_cta_cycles(t, chunk, std::min(1 << lg, h->nl), r64, batch ? 8 : 16);
+    if (batch) return ctas * (kSolveFixedCycles / 4 + one) + 32 * one;
+    return (double)((ctas + sms - 1) / sms) * one + (double)((ctas + 2 * sms - 1) / (2 * sms)) * kSolveFixedCycles;
+}
+
+// The model's choice for the Krylov-precision and the state solves; false if nothing fits.
+bool set_inv_chunks(gbprop_ctx* h, int batch) {
+    for (int dir = 0; dir < 2; ++dir)
+        for (int state = 0; state < 2; ++state) {
+            InvTab& t = state ? h->sinv[dir] : h->inv[dir];
+            const int r64 = state || h->prec == GBPROP_FP64;
+            t.warps = batch ? 8 : 16;
+            InvTab best = t;
+            double best_cost = -1.0;
+            for (int nch = 1, prev = 0; nch <= t.n; nch += 1 + nch / 16) {
+                const int chunk = chunk_of(t.n, nch);
+                if (chunk == prev) continue;
+                prev = chunk;
+                for (int lg = 0; lg <= 4 && (lg == 0 || (1 << (lg - 1)) < h->nl); ++lg) {
+                    const double c = solve_cost(h, t, chunk, lg, r64, batch);
+                    if (best_cost >= 0.0 && c >= best_cost) continue;
+                    if (!set_solve_shape(t, chunk, lg, r64)) break;
+                    best = t;
+                    best_cost = c;
+                }
+                if (chunk <= 16) break;
+            }
+            if (best_cost < 0.0) return false;
+            t = best;
+            if (!state) continue;
+            // in place: the best shape of one chunk where it costs less than the copy it saves (3 us)
+            h->pinv[dir] = t;
+            InvTab one = t;
+            best_cost += 6000.0;
+            for (int lg = 0; lg <= 4 && (lg == 0 || (1 << (lg - 1)) < h->nl); ++lg) {
+                const int chunk = chunk_of(t.n, 1);
+                const double c = solve_cost(h, t, chunk, lg, r64, batch);
+                if (c >= best_cost) continue;
+                if (!set_solve_shape(one, chunk, lg, r64)) break;
+                h->pinv[dir] = one;
+                best_cost = c;
+            }
+        }
+    return true;
 }
 
 // Triangular solve of the Krylov precision: FP64-accurate (FP32 solve + FP64 refinement)
@@ -630,10 +682,11 @@ cudaError_t ksolve(gbprop_ctx* h, int dir, const void* in, int in_prec, void* ou
 }
 
 // FP64-accurate solve of the state transforms (both precisions).
-cudaError_t ssolve(gbprop_ctx* h, int dir, const void* in, int in_prec, void* out, int out_prec) {
+// leave = 1: psi stays as it was when a step gave up on a wait
+cudaError_t ssolve(gbprop_ctx* h, int dir, const void* in, int in_prec, void* out, int out_prec, int leave = 0) {
     if (h->inv_ok)
-        return launch_solve_inv(h->inv[dir], h->nl, 1, in, in_prec, out, out_prec, nullptr, 0, h->d_ctrl, dir, 0, 0,
-                                h->stream);
+        return launch_solve_inv(h->sinv[dir], h->nl, 1, in, in_prec, out, out_prec, nullptr, 0, h->d_ctrl, dir, 0,
+                                leave ? 2 : 0, h->stream);
     return launch_solve_ir(&h->t32.tab[dir], h->d_ud_phys, h->nl, in, in_prec, out, out_prec, nullptr, 0, h->d_ctrl, 0,
                            0, h->stream);
 }
@@ -657,7 +710,7 @@ gbprop_status enqueue_enter(gbprop_ctx* h, void* psi, cudaStream_t s) {
 gbprop_status enqueue_leave(gbprop_ctx* h, void* psi, cudaStream_t s) {
     cudaStream_t keep = h->stream;
     h->stream = s;
-    cudaError_t e = ssolve(h, 0, h->d_x, 0, psi, h->kprec());
+    cudaError_t e = ssolve(h, 0, h->d_x, 0, psi, h->kprec(), 1);
     h->stream = keep;
     if (e != cudaSuccess) return fail(GBPROP_ECUDA, std::string("ssolve: ") + cudaGetErrorString(e));
     tick(h, GBPROP_PHASE_SOLVE);
@@ -970,24 +1023,29 @@ gbprop_status gbprop_finalize(gbprop_handle h) {
                 t.w = hi[dir].w;
                 t.npad = hi[dir].npad;
                 t.refine = std::max(hi[0].refine, hi[1].refine);
-                float *dm, *duh, *dul;
+                t.ks = hi[dir].ks;
+                const int up = inv_upitch(h->kd);
+                std::vector<double> u((size_t)t.npad * up, 0.0);
+                std::vector<float2> uf(u.size(), make_float2(0.f, 0.f));
+                for (int d = 0; d <= h->kd; ++d)
+                    for (int q = 0; q < t.npad; ++q) {
+                        const double v = hi[dir].u[(size_t)d * t.npad + q];
+                        const float f = (float)v;
+                        u[(size_t)q * up + d] = v;
+                        uf[(size_t)q * up + d] = make_float2(f, (float)(v - (double)f));
+                    }
+                unsigned short* dm;
                 double* du;
-                std::vector<float> uh(hi[dir].u.size()), ul(hi[dir].u.size());
-                for (size_t k = 0; k < uh.size(); ++k) {
-                    uh[k] = (float)hi[dir].u[k];
-                    ul[k] = (float)(hi[dir].u[k] - (double)uh[k]);
-                }
-                if ((st = h->upload(&dm, hi[dir].m))) return st;
-                if ((st = h->upload(&du, hi[dir].u))) return st;
-                if ((st = h->upload(&duh, uh))) return st;
-                if ((st = h->upload(&dul, ul))) return st;
-                t.m = dm;
+                float2* duf;
+                if ((st = h->upload(&dm, hi[dir].mf))) return st;
+                if ((st = h->upload(&du, u))) return st;
+                if ((st = h->upload(&duf, uf))) return st;
+                t.mf = dm;
                 t.u = du;
-                t.uh = duh;
-                t.ul = dul;
+                t.uf = duf;
+                h->sinv[dir] = t;
             }
-            set_inv_chunks(h, true);
-            h->inv_ok = true;
+            h->inv_ok = set_inv_chunks(h, 0);
         }
     }
     HostBandOp ho = build_band_op(h);
@@ -1166,7 +1224,17 @@ gbprop_status gbprop_solve_sqrt_overlap(gbprop_handle h, int conj, void* psi) {
     if (!psi) return fail(GBPROP_EINVAL, "null wavefunction");
     const int kp = h->kprec();
     GB_CUDA(h->begin());
-    GB_LAUNCH(ssolve(h, conj ? 1 : 0, psi, kp, psi, kp));
+    const int dir = conj ? 1 : 0;
+    if (!h->inv_ok || h->pinv[dir].nchunks == 1) {
+        // a CTA has read its whole rows before it writes them
+        GB_LAUNCH(h->inv_ok ? launch_solve_inv(h->pinv[dir], h->nl, 1, psi, kp, psi, kp, nullptr, 0, h->d_ctrl, dir, 0, 0,
+                                               h->stream)
+                            : ssolve(h, dir, psi, kp, psi, kp));
+    } else {
+        // with several chunks a row's halo is its neighbour's output: not in place
+        GB_LAUNCH(ssolve(h, dir, psi, kp, h->d_y, kp));
+        GB_CUDA(cudaMemcpyAsync(psi, h->d_y, (size_t)h->N * h->kelem(), cudaMemcpyDeviceToDevice, h->stream));
+    }
     GB_CUDA(h->end());
     return GBPROP_OK;
 }
@@ -1356,22 +1424,37 @@ gbprop_status gbprop_autotune(gbprop_handle h, int* variant) {
         if (ms < best_ms) { best_ms = ms; best = v; }
     }
     // radial chunking of the overlap-factor solves (one problem spread over the GPU): time the
-    // Krylov-precision solve of each direction for 1..8 chunks and keep the fastest (batches keep
-    // the fewest chunks, other problems fill the GPU)
-    if (h->inv_ok && h->expm_max_cluster > 1) {
+    // Krylov-precision solve of each direction around the cost model's choice and keep the fastest
+    // (batches keep the model's, other problems fill the GPU)
+    if (h->inv_ok && !h->in_batch) {
         // finite non-zero input (0x3f bytes): a zero right-hand side ends the refinement early
         GB_CUDA(cudaMemsetAsync(h->d_s, 0x3f, (size_t)h->N * h->kelem(), s));
         for (int dir = 0; dir < 2; ++dir) {
             const InvTab keep = h->inv[dir];
-            if (pin_c[dir] > 0) {
-                if (!set_inv_chunk_count(h, dir, pin_c[dir])) h->inv[dir] = keep;
-                continue;
+            const int r64 = h->prec == GBPROP_FP64;
+            // candidates: the shapes of the shortest modelled times
+            std::vector<std::pair<double, std::pair<int, int>>> cand;
+            for (int nch = 1, prev = 0; nch <= h->nr; ++nch) {
+                const int chunk = chunk_of(h->nr, nch);
+                if (chunk == prev) continue;
+                prev = chunk;
+                for (int lg = 0; lg <= 4 && (lg == 0 || (1 << (lg - 1)) < h->nl); ++lg)
+                    if (pin_c[dir] > 0 ? chunk == chunk_of(h->nr, pin_c[dir]) : true)
+                        cand.push_back({solve_cost(h, keep, chunk, lg, r64, 0), {chunk, lg}});
+                if (chunk <= 16) break;
             }
+            std::sort(cand.begin(), cand.end());
+            const size_t most = pin_c[dir] > 0 ? 1 : 8;
             InvTab best_t = keep;
             float best_s = 1e30f;
-            for (int nch = 1; nch <= 8; ++nch) {
-                if (nch > 1 && (h->nr + nch - 1) / nch < 32) break;
-                if (!set_inv_chunk_count(h, dir, nch)) continue;
+            size_t timed = 0;
+            for (size_t q = 0; q < cand.size() && timed < most && cand[q].first <= 1.4 * cand[0].first; ++q) {
+                if (!set_solve_shape(h->inv[dir], cand[q].second.first, cand[q].second.second, r64)) continue;
+                ++timed;
+                if (pin_c[dir] > 0) {
+                    best_t = h->inv[dir];
+                    break;
+                }
                 for (int k = 0; k < 3; ++k) GB_LAUNCH(ksolve(h, dir, h->d_s, kp, h->d_y, kp, nullptr, kp, 0, 0));
                 GB_CUDA(cudaEventRecord(e0, s));
                 for (int k = 0; k < 10; ++k) GB_LAUNCH(ksolve(h, dir, h->d_s, kp, h->d_y, kp, nullptr, kp, 0, 0));
@@ -1846,18 +1929,35 @@ gbprop_status gbprop_batch_create(gbprop_batch* out, const gbprop_handle* proble
         delete b;
         return fail(GBPROP_ECUDA, std::string("batch stream/event creation: ") + cudaGetErrorString(e));
     }
-    for (gbprop_handle h : b->hs) {
-        h->expm_max_cluster = 1;        // other problems fill the GPU: one CTA per exponential
-        if (h->inv_ok) set_inv_chunks(h, false);
-        // Gram-Schmidt of a complex64 basis: the cooperative form on a grid sized to the problem
-        // (measured: mixed batch 76.0 -> 72.5 ms per step; FP64 batches keep the three-kernel form,
-        // 161 against 195 ms with it; GBPROP_CGS=separate keeps it for both)
+    // The exponential of a member spreads over a cluster while the batch leaves SMs free for it: with 16
+    // CTAs against one CTA per problem a batch step took 0.75-0.95 of the time for 4 to 48 problems,
+    // 1.00 (FP64) and 1.05 (mixed) for 96, 1.16 and 1.07 for 256.
+    const int expm_cluster = count <= 64 ? 16 : 1;
+    // Gram-Schmidt of a member: the cooperative form on a grid sized to the problem.  A complex64 basis
+    // always takes it (mixed batch of 256: 76.0 -> 72.5 ms per step).  An FP64 basis takes it where the grid
+    // is at most a quarter of the SMs, or the members' grids together at most twice the SMs -- larger ones
+    // wait for free SMs: a step of 4 x (65 x 1500) took 4.75 ms with it and 4.98 with three kernels, of 20 x
+    // (33 x 420) 4.24 and 4.92, of 96 x (40 x 500) 21.7 and 23.5, but of 12 x (65 x 1500) 9.04 and 7.88.
+    // (GBPROP_CGS=separate keeps the three-kernel form.)
+    const char* cgs_env = std::getenv("GBPROP_CGS");
+    const bool cgs_separate = cgs_env && std::strcmp(cgs_env, "separate") == 0;
+    std::vector<int> grids(count, 0), caches(count, 0);
+    long grid_sum = 0;
+    for (int p = 0; p < count; ++p) {
+        gbprop_ctx* h = b->hs[p];
+        if (cgs_separate || h->double_orth) continue;
+        grids[p] = arnoldi_cgs_grid_batch(h->kprec(), h->N, h->m, h->d_v0 != nullptr, &caches[p]);
+        grid_sum += grids[p];
+    }
+    for (int p = 0; p < count; ++p) {
+        gbprop_ctx* h = b->hs[p];
+        h->expm_max_cluster = expm_cluster;
+        h->in_batch = true;
+        if (h->inv_ok) set_inv_chunks(h, 1);
         {
-            const char* env = std::getenv("GBPROP_CGS");
-            int cache = 0;
-            const int grid = (env && std::strcmp(env, "separate") == 0) || h->double_orth || h->prec == GBPROP_FP64
-                                 ? 0
-                                 : arnoldi_cgs_grid_batch(h->kprec(), h->N, h->m, h->d_v0 != nullptr, &cache);
+            const int sms = grid_reduce_blocks();
+            const bool coop = h->prec != GBPROP_FP64 || 4 * grids[p] <= sms || grid_sum <= 2 * sms;
+            const int grid = coop ? grids[p] : 0, cache = caches[p];
             cudaGetLastError();
             if (grid > 0 && !h->d_gridbar) {
                 if (gbprop_status st = h->dalloc(&h->d_gridbar, 64)) {
@@ -1974,7 +2074,8 @@ gbprop_status gbprop_batch_destroy(gbprop_batch b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     for (gbprop_handle h : b->hs) {
         h->expm_max_cluster = 16;
-        if (h->inv_ok) set_inv_chunks(h, true);
+        h->in_batch = false;
+        if (h->inv_ok) set_inv_chunks(h, 0);
     }
     delete b;
     return GBPROP_OK;

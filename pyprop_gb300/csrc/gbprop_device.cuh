@@ -121,6 +121,20 @@ __device__ __forceinline__ float d2f_fast(double d) {
     return __uint_as_float(bits);
 }
 
+// what d2f_fast rounds off, d - (double)d2f_fast(d), to FP32 precision: the 29 mantissa bits below the
+// FP32 value as a signed integer, its exponent set by integer addition (zero below FP32's normal range)
+__device__ __forceinline__ float d2f_low(double d) {
+    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+    const int e = (int)((hi >> 20) & 0x7ffu);
+    const unsigned fm = lo >> 29, rem = lo & 0x1fffffffu;
+    const unsigned up = (rem > 0x10000000u) | ((rem == 0x10000000u) & fm & 1u);
+    const int r = (int)rem - (up ? 0x20000000 : 0);
+    const unsigned f = __float_as_uint((float)r);
+    const int fe = (int)((f >> 23) & 0xffu) + e - 1075;
+    if (r == 0 || fe <= 0 || fe >= 255) return 0.f;
+    return __uint_as_float((f + ((unsigned)(e - 1075) << 23)) ^ (hi & 0x80000000u));
+}
+
 __device__ __forceinline__ double f2d_fast(float f) {
     const unsigned u = __float_as_uint(f);
     const unsigned e = (u >> 23) & 0xffu, sign = u & 0x80000000u;
@@ -128,6 +142,16 @@ __device__ __forceinline__ double f2d_fast(float f) {
     const unsigned hi = e == 0 ? sign : (sign | (de << 20) | ((u & 0x7fffffu) >> 3));
     const unsigned lo = e == 0 ? 0u : (u & 0x7u) << 29;
     return __hiloint2double((int)hi, (int)lo);
+}
+
+// 2^e as a double, -1022 <= e <= 1023
+__device__ __forceinline__ double pow2_double(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+
+// d * 2^s by the exponent field; zero, subnormals and results below the normal range become signed zero
+__device__ __forceinline__ double scale_pow2(double d, int s) {
+    const int hi = __double2hiint(d), e = ((hi >> 20) & 0x7ff), f = e + s;
+    if (e == 0 || f <= 0) return __hiloint2double(hi & 0x80000000, 0);
+    return __hiloint2double(hi + (s << 20), __double2loint(d));
 }
 
 // ---------------------------------------------------------------------------
@@ -153,6 +177,13 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  :: "r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
+
+// 16-byte asynchronous copy global -> shared of one thread, and its wait for all of them
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" :: "l"(p)); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Bounded wait for phase 0 of the mbarrier; false when the poll limit was reached.
 __device__ __forceinline__ bool mbar_wait0(unsigned long long* bar, long limit = kInvWaitLimit) {
@@ -247,36 +278,51 @@ __device__ __forceinline__ void warp_pair_sum(float& h, float& l) {
     }
 }
 
-// beta = ||w|| of the next basis vector from the cooperative Gram-Schmidt kernel's per-CTA
-// ||w||^2 partials, summed by one warp in a fixed order (the same beta in every CTA that
-// calls it).  PAIRS: FP32-pair partials (float4 hi, lo, -, -) of the complex64 form, else one
-// double per CTA.  Whole warp; returns beta in every lane.
-template <bool PAIRS>
+// ||w||^2 of the next basis vector from the complex64 Gram-Schmidt kernel's per-CTA partials
+// (float4 hi, lo, -, -), summed by one warp in a fixed order; a normalised FP32 pair in every lane.
+__device__ __forceinline__ float2 gs_norm2_pair(const float4* p, int G) {
+    const int lane = threadIdx.x & 31;
+    float a = 0.f, c = 0.f;
+    for (int g0 = lane; g0 < G; g0 += 8 * 32) {
+        float4 t[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int g = g0 + 32 * u;
+            t[u] = g < G ? __ldcg(p + g) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc_pair(a, c, t[u].x, t[u].y);
+    }
+    warp_pair_sum(a, c);
+    float s, e;
+    two_sum(a, c, s, e);
+    return make_float2(s, e);
+}
+
+// 1 / sqrt(th + tl) as an FP32 pair: the hardware estimate y and one Newton step whose residual
+// 1 - t y^2 is formed error-free, with the second-order term (relative error below 2^-45)
+__device__ __forceinline__ float2 inv_sqrt_pair(float th, float tl) {
+    const float y = rsqrtf(th);
+    const float p = __fmul_rn(y, y), pe = __fmaf_rn(y, y, -p);
+    const float q = __fmul_rn(th, p), qe = __fmaf_rn(th, p, -q);
+    const float r = __fsub_rn(__fsub_rn(__fsub_rn(1.f, q), qe), __fmaf_rn(tl, p, __fmul_rn(th, pe)));
+    const float d = __fmul_rn(y, __fmaf_rn(__fmul_rn(0.375f, r), r, __fmul_rn(0.5f, r)));
+    float s, e;
+    two_sum(y, d, s, e);
+    return make_float2(s, e);
+}
+
+// beta = ||w|| of the next basis vector from the FP64 cooperative Gram-Schmidt kernel's per-CTA
+// ||w||^2 partials (one double per CTA), summed by one warp in a fixed order (the same beta in every
+// CTA that calls it).  Whole warp; returns beta in every lane.
 __device__ __forceinline__ double gs_beta(const void* part, int G) {
     const int lane = threadIdx.x & 31;
-    if constexpr (PAIRS) {
-        const float4* p = reinterpret_cast<const float4*>(part);
-        float a = 0.f, c = 0.f;
-        for (int g0 = lane; g0 < G; g0 += 8 * 32) {
-            float4 t[8];
+    const double* p = reinterpret_cast<const double*>(part);
+    double t = 0.0;
+    for (int g = lane; g < G; g += 32) t += __ldcg(p + g);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int g = g0 + 32 * u;
-                t[u] = g < G ? __ldcg(p + g) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) acc_pair(a, c, t[u].x, t[u].y);
-        }
-        warp_pair_sum(a, c);
-        return sqrt((double)a + (double)c);
-    } else {
-        const double* p = reinterpret_cast<const double*>(part);
-        double t = 0.0;
-        for (int g = lane; g < G; g += 32) t += __ldcg(p + g);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        return sqrt(t);
-    }
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return sqrt(t);
 }
 
 // Records beta of the next basis vector (pamp.h:330-345; happy breakdown below sqrt(eps),

@@ -39,20 +39,39 @@ template <typename T> struct SolveTab {
 // are upper triangular:  U~(q, q+d), d = 0..kd  and  M(q, q+j) ~ U~^-1(q, q+j), j = 0..w.
 // U^-1 of a B-spline overlap factor decays geometrically away from the diagonal, so
 // w is chosen (on the host) where the dropped part is below 2^-26 of the kept one.
-//   m  (j*npad + q)  FP32, zero where q + j >= n;  npad = n rounded up to 4
-//   u  (d*npad + q)  FP64, zero where q + d >= n
-// Each CTA owns `chunk` radial elements (a multiple of 4) of one row and recomputes the
-// halo its refinement passes need; stage = 1 copies the chunk's slice of m into shared memory
-// with bulk asynchronous copies (16-byte aligned: q0, npad multiples of 4).
+//   mf  bfloat16, blocks of sixteen outputs, ks steps of sixteen columns (16 ks >= w + 16, a multiple
+//       of kSolveFrags steps, which the kernel loads at once) and three parts whose sum is the FP32
+//       M(r, c), in the fragment order of mma.m16n8k16: entry (((B*ks + s)*3 + part)*32 + lane)*8 + e with
+//       r = 16B + lane/4 + 8 (e/2 % 2), c = 16B + 16s + 2 (lane%4) + e%2 + 8 (e/4); zero outside the band
+//       and the matrix
+//   u   q*inv_upitch(kd) + d  FP64 (an odd row length: a warp's rows lie in different banks), zero
+//       where q + d >= n; npad rows, npad = n rounded up to 4
+//   uf  the same entries split into FP32 pairs u = uf.x + uf.y, for the error-free residuals
+// Each CTA owns `chunk` radial elements (a multiple of 16) of `rg` rows and recomputes the halo its
+// refinement passes need; stage = 1 copies the chunk's slices of U~ into shared memory (16-byte
+// asynchronous copies: q0 and npad are multiples of 4).
+constexpr int kSolveFrags = 5;
+__host__ __device__ constexpr int inv_upitch(int kd) { return (kd + 1) | 1; }
+
+// Byte offsets of a solve CTA's shared memory: U~ slices (staged) | right-hand side (FP64 complex, or
+// complex FP32 pairs) | FP64 iterate | residual in bfloat16 parts | FP32 first iterate.
+struct InvLayout {
+    int u, uf, b, x, r16, x0, bytes;
+};
+
 struct InvTab {
     int n, kd, w, npad;
+    int ks;                 // k steps of a block
+    int lg;                 // log2 of the rows per CTA
+    int warps;              // worker warps per CTA (8 or 16)
     int chunk, nchunks;
-    int refine;             // FP64-residual refinement passes of the FP64-accurate solve
+    int refine;             // refinement passes of the FP64-accurate solve
     int stage;
-    const float* m;
+    int pq, px, pd, pb, pl; // shared-memory pitches (inv_shape)
+    InvLayout ly;
+    const unsigned short* mf;
     const double* u;
-    const float* uh;        // u split into FP32 pairs u = uh + ul (same layout), for the
-    const float* ul;        // error-free residual of the complex64 solve
+    const float2* uf;
 };
 
 // Region of the CTA whose chunk starts at q0, for P refinement passes: cl elements written,
@@ -66,31 +85,38 @@ __host__ __device__ inline void inv_region(int n, int q0, int chunk, int P, int 
     *RB = rb < left ? rb : left;
 }
 
-// Shared-memory bytes of that CTA: b | x, r (FP64, refined solve only) | M slice (staged; read
-// three times) | r32 | x0 (FP32 first iterate, refined solve only).  U~ is read once per
-// residual pass and comes through L2.
-__host__ __device__ inline size_t inv_smem_bytes(int n, int q0, int chunk, int P, int w, int kd, int stage, int r64) {
+// Shared-memory pitches and offsets of a solve CTA (the same for every chunk, sized by the first):
+// residual entries per plane (8 mod 64: the eight planes and four pairs of columns of a B fragment lie
+// in 32 banks), x0 complex64 per row (4 mod 16) and x complex128 per row (2 mod 8), whose four rows by
+// four or two columns an accumulator fragment stores together, b complex per row.
+inline void inv_shape(InvTab& t, int r64) {
     int cl, R0, RB;
-    inv_region(n, q0, chunk, P, w, kd, &cl, &R0, &RB);
-    const int R0p = (R0 + 3) & ~3;
-    size_t b = (size_t)RB * 16;
-    if (r64) b += (size_t)R0 * 16 + (size_t)RB * 16;
-    if (stage) b += (size_t)(w + 1) * R0p * 4;
-    b += (size_t)(R0 + w + 2) * 8;                  // r32 with the padding of the paired M product
-    if (r64) b += (size_t)R0 * 8;
-    return b;
-}
-
-// Shared memory of the complex64 (mixed-path) solve with one refinement:
-// M slice | uh, ul slices (staged) | b hi, b lo | x0 | r32.
-__host__ __device__ inline size_t inv_smem_bytes_mixed(int n, int q0, int chunk, int w, int kd, int stage) {
-    int cl, R0, RB;
-    inv_region(n, q0, chunk, 1, w, kd, &cl, &R0, &RB);
-    const int R0p = (R0 + 3) & ~3;
-    size_t b = 0;
-    if (stage) b += (size_t)(w + 1) * R0p * 4 + (size_t)2 * (kd + 1) * R0p * 4;
-    b += (size_t)RB * 16 + (size_t)((R0 + 1) & ~1) * 8 + (size_t)(R0 + w + 2) * 8;
-    return b;
+    const int P = r64 ? t.refine : 1;
+    inv_region(t.n, 0, t.chunk, P, t.w, t.kd, &cl, &R0, &RB);
+    const int r0 = (R0 + 15) & ~15;
+    const int d = P >= 2 ? cl + (P - 1) * (t.w + t.kd) : R0;      // the FP64 iterate starts after an FP32-pair pass
+    const int rd = ((d < R0 ? d : R0) + 15) & ~15;
+    const int vq = r0 + 16 * t.ks > RB ? r0 + 16 * t.ks : RB;
+    t.pq = ((vq - 8 + 63) & ~63) + 8;
+    t.px = ((r0 + t.kd - 4 + 15) & ~15) + 4;
+    t.pd = ((rd + t.kd - 2 + 7) & ~7) + 2;
+    t.pb = RB;
+    const int rows = 1 << t.lg, ub = ((R0 + 3) & ~3) * inv_upitch(t.kd) * 8;
+    int o = 0;
+    t.ly.u = o;
+    if (t.stage && r64) o += ub;
+    t.ly.uf = o;
+    if (t.stage) o += ub;
+    t.ly.b = o;
+    o += rows * t.pb * 16;
+    t.ly.x = o;
+    if (r64) o += rows * t.pd * 16;
+    t.ly.r16 = o;
+    t.pl = 2 * (rows < 4 ? 4 : rows) * t.pq;         // whole groups of eight planes
+    o += 3 * t.pl * 2;                               // (a multiple of 16 bytes: 8 planes, pq a multiple of 8)
+    t.ly.x0 = o;
+    o += rows * t.px * 8;
+    t.ly.bytes = o;
 }
 
 // Term list of the tensor-potential matvec, grouped by destination row l:
@@ -181,10 +207,11 @@ cudaError_t launch_solve_ir(const void* tabf, const double* udp, int nrows, cons
                             int out_prec, void* vstore, int v_prec, const Ctrl* ctrl, int scale_mode, int check_broken,
                             cudaStream_t s);
 // Solve through the banded approximate inverse of the overlap factor (see InvTab):
-// x = M b in FP32, then `refine` passes x += M (b - U~ x) with FP64 residuals when
+// x = M b in FP32, then `refine` passes x += M (b - U~ x), the last with FP64 residuals when
 // refine64 is set (FP64-accurate result).  refine64 = 0 is the complex64 solve of the mixed
 // path's Krylov basis: one refinement whose residual is formed with error-free FP32 products
-// and sums, complex64 output.  Grid: (tab.nchunks, nrows); arguments as launch_solve.
+// and sums, complex64 output.  in and out must not overlap (a chunk's halo is read by its
+// neighbour).  check_broken 2: nothing is written once ctrl->wait_timeout is set.  Grid: (tab.nchunks, row groups); arguments as launch_solve.
 // v0s (complex64 solve of the FP64 first vector only, may be null) receives the scaled input
 // split into FP32 pairs, float4 (re_hi, im_hi, re_lo, im_lo) per element.  bpart (scale_mode
 // 1, may be null): the cooperative Gram-Schmidt kernel's bG per-CTA ||w||^2 partials (double,

@@ -1,14 +1,14 @@
 // Banded triangular solves along r (ztbsv 'U','N' / 'U','C' in the reference,
 // piram/piram/blitzblas.h:454-487, called from overlapmatrix.cpp:137-229):
-//   * k_solve_inv   -- banded approximate inverse of the overlap factor applied in FP32
-//                      with FP64-residual refinement (the runtime's default);
+//   * k_solve_rows  -- banded approximate inverse of the overlap factor applied in FP32
+//                      with refinement from FP32-pair and FP64 residuals (the runtime's default);
 //   * k_solve_ir    -- FP32 block back-substitution + FP64 refinement (fallback for
 //                      factors whose inverse decays too slowly);
 //   * k_solve       -- the block back-substitution in one precision.
 #include "gbprop_internal.h"
 #include "gbprop_device.cuh"
 
-#include <algorithm>
+#include <cfloat>
 #include <cmath>
 
 namespace gbprop {
@@ -359,559 +359,532 @@ cudaError_t launch_solve_ir(const void* tabf, const double* udp, int nrows, cons
 // ---------------------------------------------------------------------------
 // solve through the banded approximate inverse (all threads busy, no recursion)
 // ---------------------------------------------------------------------------
-// CTA (chunk c, row l) produces x on q in [q0, q0 + cl), q0 = c * chunk.  With P
-// refinement passes, pass k (0..P) updates x on [q0, q0 + R_k), R_k = cl + (P-k)(w+kd):
-//     r = b - U~ x          (FP64; pass 0: r = b, x = 0)
-//     x += 2^e * M (2^-e r) (FP32 products and sums; 2^-e only when max|r| leaves the
-//                            comfortable FP32 exponent range)
-// x on R_k needs r on R_k + w, which needs the previous x on R_k + w + kd = R_{k-1}, so
-// the chunk's halo is recomputed instead of exchanged.  Every element of the region is
-// independent inside a pass: one thread per element, two barriers per pass.  The chunk's
-// slices of M and U~ arrive by bulk asynchronous copies (one mbarrier) while the threads
-// load the right-hand side.
-constexpr int kInvThreads = 512;
-// x (+)= M r32 for the elements q and q + 1 (q even; r32 16-byte aligned and readable up to
-// q + w + 1): FP32 products, two independent chains per component.  Every pair of r32
-// values is one 16-byte load and every pair of M entries one 8-byte load, each used for
-// both outputs -- 3 loads per 8 FMAs instead of 8.  With t = j for element q and t = j + 1
-// for element q + 1, r32[q + t] meets M[t][q] and M[t-1][q+1].
-template <bool STAGE>
-__device__ __forceinline__ float2 inv_m2(const float* mrow, size_t mstride, int t) {
-    const float2* p = reinterpret_cast<const float2*>(mrow + (size_t)t * mstride);
-    return STAGE ? *p : __ldg(p);
+// CTA (chunk c, row group g) produces x on q in [q0, q0 + cl), q0 = c * chunk, for up to `rg`
+// angular rows.  With P refinement passes, pass k (0..P) forms M r on [q0, q0 + R_k),
+// R_k = cl + (P-k)(w+kd), and adds it to x:
+//     r = b                 (pass 0, FP32)
+//     r = b - U~ x          (later passes)
+// x on R_k needs r on R_k + w, which needs the previous x on R_k + w + kd = R_{k-1}, so the
+// chunk's halo is recomputed instead of exchanged.
+//   * FP64-accurate solve (R64): x0 is exact in FP32, so the first residual is formed from FP32
+//     pairs (U~ = uh + ul, b = bh + bl; error-free products and sums); the last ones are in FP64.
+//   * complex64 solve of the mixed path's basis: P = 1 with the FP32-pair residual.  The
+//     refinement makes the operator seen by the basis U^-1 to ~1e-13 (the FP32 band of M alone
+//     perturbs it by ~1e-7, which shifts high eigenvalues systematically).  A double2 operand (the
+//     FP64 first vector) is used as hi + lo, a complex64 operand as stored, so the solve acts on
+//     exactly the vector kept in the basis.
+//
+// U is real and the same for every row, so the rows' real and imaginary parts are columns of one
+// right-hand side and the band product of a CTA is a banded matrix times a (radial) x (2 rows)
+// matrix: it runs on the tensor cores (mma.sync m16n8k16, bfloat16 operands, FP32 accumulation), M
+// and r each split exactly into three bfloat16 parts, six products (the other three are below FP32's
+// resolution).  A warp owns sixteen outputs of eight columns; M comes in fragment order (InvTab), one
+// 16-byte load per lane, part and k step, through L1 and L2: a CTA uses an entry once per pass.  A
+// lane's accumulators are one row's real and imaginary part of two outputs.  (Two TF32 parts, three
+// products, take as many instructions with the splitting of M and leave 2^-22 instead of 2^-24 of the
+// product: states that fall off towards the origin by tens of orders keep the error of that as noise
+// in the operator's stiff modes, 50 times more in a step of the 64 x 1000 hydrogen operator.)
+// What bounds it: the FP64 residual, 2 (kd+1) FP64 warp instructions per 32 complex elements at 16 SM
+// cycles each, on the chunk and w halo elements; then the latency of the barrier-separated phases.
+// The form before this one gave a thread two complex outputs of one row and fed FP32 FMAs from shared
+// memory at 8 bytes per FMA per lane, which bound it.  (Sharing an M entry among the lanes of all rows
+// instead does not help FMAs: a broadcast costs the register-side bandwidth of the loads all the same.)
+//
+// beta of an Arnoldi vector (the norm partials of the previous Gram-Schmidt launch) is formed by a
+// warp of its own.  The FP64-accurate solve runs on the unscaled vector meanwhile and multiplies v
+// and x by 1/beta when it stores them; the complex64 solve needs v rounded first and waits for an
+// FP32-pair reciprocal square root.
+//
+// Worker warps: 16 for a problem alone (one CTA per SM; its phases are latency-bound), 8 inside a
+// batch, where two or three CTAs of different problems share an SM (InvTab::warps).
+constexpr int kRowWarps = 16;                        // most worker warps
+constexpr int kRowBlock = 32 * kRowWarps + 32;       // + the warp that forms 1/beta
+
+__device__ __forceinline__ void worker_sync(int nw) { asm volatile("bar.sync 1, %0;" :: "r"(32 * nw) : "memory"); }
+
+template <bool SMEM, typename T> __device__ __forceinline__ T row_ld(const T* p) { return SMEM ? *p : __ldg(p); }
+
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint4& a, unsigned b0, unsigned b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
 }
 
-template <bool STAGE>
-__device__ __forceinline__ float4 inv_apply2(const float* mrow, size_t mstride, const float2* r32, int q, int w) {
-    const float4* r4 = reinterpret_cast<const float4*>(r32 + q);
-    float a0r = 0.f, a0i = 0.f, b0r = 0.f, b0i = 0.f;   // element q: even / odd t
-    float a1r = 0.f, a1i = 0.f, b1r = 0.f, b1i = 0.f;   // element q + 1
-    float pm = 0.f;                                     // M[t-1][q+1] (none at t = 0)
-    int t = 0;
-    for (; t + 1 <= w; t += 2) {
-        const float4 rr = r4[t >> 1];                   // r[q+t], r[q+t+1]
-        const float2 m0 = inv_m2<STAGE>(mrow, mstride, t), m1 = inv_m2<STAGE>(mrow, mstride, t + 1);
-        a0r = fmaf(m0.x, rr.x, a0r); a0i = fmaf(m0.x, rr.y, a0i);
-        a1r = fmaf(pm, rr.x, a1r);   a1i = fmaf(pm, rr.y, a1i);
-        b0r = fmaf(m1.x, rr.z, b0r); b0i = fmaf(m1.x, rr.w, b0i);
-        b1r = fmaf(m0.y, rr.z, b1r); b1i = fmaf(m0.y, rr.w, b1i);
-        pm = m1.y;
-    }
-    if (t <= w) {                                       // w even: t = w
-        const float4 rr = r4[t >> 1];
-        const float2 m0 = inv_m2<STAGE>(mrow, mstride, t);
-        a0r = fmaf(m0.x, rr.x, a0r); a0i = fmaf(m0.x, rr.y, a0i);
-        a1r = fmaf(pm, rr.x, a1r);   a1i = fmaf(pm, rr.y, a1i);
-        b1r = fmaf(m0.y, rr.z, b1r); b1i = fmaf(m0.y, rr.w, b1i);
-    } else {                                            // w odd: t = w + 1
-        const float2 rl = r32[q + t];
-        a1r = fmaf(pm, rl.x, a1r); a1i = fmaf(pm, rl.y, a1i);
-    }
-    return make_float4(a0r + b0r, a0i + b0i, a1r + b1r, a1i + b1i);
-}
-
-template <int KD, bool R64, bool STAGE, typename TI, typename TO, typename TV>
-__global__ void __launch_bounds__(kInvThreads) k_solve_inv(InvTab tab, const TI* __restrict__ in,
-                                                           TO* __restrict__ out, TV* __restrict__ vstore,
-                                                           Ctrl* __restrict__ ctrl, int dir, int scale_mode,
-                                                           int check_broken, const double* __restrict__ bpart,
-                                                           int bG) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ unsigned s_red[kInvThreads / 32];
-    __shared__ __align__(8) unsigned long long s_bar;
-    const int n = tab.n, w = tab.w, P = R64 ? tab.refine : 0;
-    const int l = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int q0 = blockIdx.x * tab.chunk;
-    int cl, R0, RB;
-    inv_region(n, q0, tab.chunk, P, w, KD, &cl, &R0, &RB);
-    const int R0p = (R0 + 3) & ~3;
-    // carve shared memory (see inv_smem_bytes)
-    unsigned char* sp = smem_raw;
-    double2* bq = reinterpret_cast<double2*>(sp);
-    sp += (size_t)RB * 16;
-    double2* xq = reinterpret_cast<double2*>(sp);
-    double2* rq = xq + R0;
-    if (R64) sp += (size_t)R0 * 16 + (size_t)RB * 16;
-    float* Ms = reinterpret_cast<float*>(sp);
-    if (STAGE) sp += (size_t)(w + 1) * R0p * 4;
-    float2* r32 = reinterpret_cast<float2*>(sp);     // 16-byte aligned; 2 slots of padding
-    sp += (size_t)(R0 + w + 2) * 8;
-    float2* x0f = reinterpret_cast<float2*>(sp);     // FP32 first iterate (exact in FP32)
-
-    const float* Mg = tab.m + q0;
-    const double* Ug = tab.u + q0;
-    const float* Uhg = tab.uh + q0;
-    const float* Ulg = tab.ul + q0;
-    if (STAGE) {
-        // one thread arms the barrier with the byte count and issues one bulk copy per
-        // diagonal (rows of R0p elements: sizes and addresses are multiples of 16 bytes)
-        if (tid == 0) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_bar)) : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-        __syncthreads();                               // barrier initialised before anyone polls it
-        if (tid == 0) {
-            const unsigned mrow = (unsigned)R0p * 4;
-            const unsigned bytes = (unsigned)(w + 1) * mrow;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                         :: "r"(smem_u32(&s_bar)), "r"(bytes) : "memory");
-            for (int j = 0; j <= w; ++j) bulk_g2s(Ms + (size_t)j * R0p, Mg + (size_t)j * tab.npad, mrow, &s_bar);
-        }
-    }
-    // the band of M is constant and is staged before the wait; everything below reads what
-    // earlier kernels wrote
-    pdl_wait();
-    if (check_broken && ctrl->broken) {
-        if (STAGE) mbar_wait0(&s_bar);             // copies in flight land before exit
-        return;
-    }
-    const float* mbase = STAGE ? Ms : Mg;
-    const size_t mstride = STAGE ? (size_t)R0p : (size_t)tab.npad;
-    const double* ubase = Ug;
-    const float* uhb = Uhg;
-    const float* ulb = Ulg;
-    const size_t ustride = (size_t)tab.npad;
-    const size_t base = (size_t)l * n;
-
-    {
-        // late: 1/beta comes from the Gram-Schmidt kernel's norm partials -- warp 0 forms it
-        // while the other warps load the right-hand side, which is scaled afterwards
-        const bool late = scale_mode && bpart;
-        const double sc = scale_mode && !late ? ctrl->inv_beta : 1.0;
-        __shared__ double s_ibeta;
-        __shared__ int s_brk;
-        if (late && warp == 0) {
-            const double beta = gs_beta<false>(bpart, bG);
-            if (lane == 0) {
-                s_brk = gs_record_beta(ctrl, beta, blockIdx.x == 0 && blockIdx.y == 0);
-                s_ibeta = 1.0 / beta;
-            }
-        }
-        const int t0 = late ? tid - 32 : tid, tstep = late ? kInvThreads - 32 : kInvThreads;
-        if (t0 >= 0)
-            for (int q = t0; q < RB; q += tstep) {
-                const int p = dir ? (n - 1 - (q0 + q)) : (q0 + q);
-                const TI t = in[base + p];
-                double2 b = make_double2((double)t.x, (double)t.y);
-                if (scale_mode && !late) { b.x *= sc; b.y *= sc; }
-                if (vstore && q < cl && !late) vstore[base + p] = conv<TV>(b);
-                bq[q] = b;
-                if (q < R0) xq[q] = make_double2(0.0, 0.0);
-            }
-        if (late) {
-            __syncthreads();
-            if (s_brk) {                               // uniform: the same beta in every CTA
-                if (STAGE) mbar_wait0(&s_bar);
-                return;
-            }
-            const double ib = s_ibeta;
-            for (int q = tid; q < RB; q += kInvThreads) {
-                double2 b = bq[q];
-                b.x *= ib;
-                b.y *= ib;
-                bq[q] = b;
-                if (vstore && q < cl) vstore[base + (dir ? (n - 1 - (q0 + q)) : (q0 + q))] = conv<TV>(b);
-            }
-        }
-        bool ok = true;
-        if (STAGE) ok = mbar_wait0(&s_bar, wait_budget(ctrl, kInvWaitLimit));
-        if (!__syncthreads_and(ok)) {
-            if (tid == 0) ctrl->wait_timeout = 1;
-            if (STAGE) mbar_wait0(&s_bar);
-            return;
-        }
-        bool x0_exact = false;                     // x after pass 0 is the FP32 vector x0f
-        for (int k = 0; k <= P; ++k) {
-            const int Rk = min(n - q0, cl + (P - k) * (w + KD));
-            const int Rr = min(n - q0, Rk + w);
-            if (k == 1 && P >= 2 && x0_exact) {
-                // first refinement: r = b - U~ x0 with x0 exact in FP32, formed with FP32 pairs
-                // (U~ = uh + ul, b = bh + bl; error-free products and sums).  Its relative error
-                // (~2^-48 |b| / |r|) is far below what this pass needs; the last pass uses an FP64
-                // residual.  No scaling: |b| has an FP32-safe exponent (checked at pass 0).
-                for (int q = tid; q < Rk + w + 2; q += kInvThreads) {
-                    float2 v = make_float2(0.f, 0.f);
-                    if (q < Rr) {
-                        float hr = 0.f, lr = 0.f, hi_ = 0.f, li = 0.f;
+// M fragments of one block, this lane's: the leading and middle parts of the first kSolveFrags k steps
+__device__ __forceinline__ void load_frags(uint4 (&a)[2 * kSolveFrags], const uint4* frag) {
 #pragma unroll
-                        for (int d = 0; d <= KD; ++d) {
-                            if (q + d < n - q0) {
-                                const float uh = __ldg(uhb + (size_t)d * ustride + q);
-                                const float ul = __ldg(ulb + (size_t)d * ustride + q);
-                                const float2 xv = x0f[q + d];
-                                acc_prod(hr, lr, uh, ul, xv.x);
-                                acc_prod(hi_, li, uh, ul, xv.y);
-                            }
-                        }
-                        const double2 b = bq[q];
-                        const float bhx = d2f_fast(b.x), bhy = d2f_fast(b.y);
-                        const float blx = d2f_fast(b.x - f2d_fast(bhx)), bly = d2f_fast(b.y - f2d_fast(bhy));
-                        float s_, e_;
-                        two_sum(bhx, -hr, s_, e_);
-                        v.x = __fadd_rn(s_, __fadd_rn(e_, __fsub_rn(blx, lr)));
-                        two_sum(bhy, -hi_, s_, e_);
-                        v.y = __fadd_rn(s_, __fadd_rn(e_, __fsub_rn(bly, li)));
-                    }
-                    r32[q] = v;
-                }
-                __syncthreads();
-                for (int q = 2 * tid; q < Rk; q += 2 * kInvThreads) {
-                    const float4 f = inv_apply2<STAGE>(mbase + q, mstride, r32, q, w);
-                    double2 x = xq[q];
-                    x.x += f2d_fast(f.x);
-                    x.y += f2d_fast(f.y);
-                    xq[q] = x;
-                    if (q + 1 < Rk) {
-                        x = xq[q + 1];
-                        x.x += f2d_fast(f.z);
-                        x.y += f2d_fast(f.w);
-                        xq[q + 1] = x;
-                    }
-                }
-                __syncthreads();
-                continue;
-            }
-            // residual r = b - U~ x (FP64, two FMA chains per component) and the max of
-            // its high words (monotone in |r|)
-            unsigned hmax = 0;
-            for (int q = tid; q < Rr; q += kInvThreads) {
-                double2 r = bq[q];
-                if (k > 0) {
-                    double ar = 0.0, ai = 0.0;
-#pragma unroll
-                    for (int d = 0; d <= KD; ++d) {
-                        if (q + d < n - q0) {
-                            const double u = __ldg(ubase + (size_t)d * ustride + q);
-                            const double2 xv = xq[q + d];
-                            if (d & 1) { ar = fma(-u, xv.x, ar); ai = fma(-u, xv.y, ai); }
-                            else { r.x = fma(-u, xv.x, r.x); r.y = fma(-u, xv.y, r.y); }
-                        }
-                    }
-                    r.x += ar;
-                    r.y += ai;
-                    rq[q] = r;
-                }
-                hmax = max(hmax, max((unsigned)__double2hiint(r.x) & 0x7fffffffu,
-                                     (unsigned)__double2hiint(r.y) & 0x7fffffffu));
-            }
-            hmax = __reduce_max_sync(0xffffffffu, hmax);
-            if (lane == 0) s_red[warp] = hmax;
-            __syncthreads();
-            hmax = 0;
-#pragma unroll
-            for (int i = 0; i < kInvThreads / 32; ++i) hmax = max(hmax, s_red[i]);
-            if (hmax == 0) break;                      // zero residual: x is exact (or b = 0)
-            const int e = (int)(hmax >> 20) - 1022;
-            const bool scaled = e < -100 || e > 100;
-            const double sdown = scaled ? ldexp(1.0, -e) : 1.0, sup = scaled ? ldexp(1.0, e) : 1.0;
-            const double2* rsrc = k > 0 ? rq : bq;
-            for (int q = tid; q < Rk + w + 2; q += kInvThreads) {
-                float2 v = make_float2(0.f, 0.f);
-                if (q < Rr) {
-                    double2 r = rsrc[q];
-                    if (scaled) { r.x *= sdown; r.y *= sdown; }
-                    v = make_float2(d2f_fast(r.x), d2f_fast(r.y));
-                }
-                r32[q] = v;
-            }
-            __syncthreads();
-            for (int q = 2 * tid; q < Rk; q += 2 * kInvThreads) {
-                const float4 f4 = inv_apply2<STAGE>(mbase + q, mstride, r32, q, w);
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    if (e == 1 && q + 1 >= Rk) break;
-                    const float2 f = e ? make_float2(f4.z, f4.w) : make_float2(f4.x, f4.y);
-                    double2 x = xq[q + e];
-                    if (scaled) { x.x = fma(f2d_fast(f.x), sup, x.x); x.y = fma(f2d_fast(f.y), sup, x.y); }
-                    else if (k == 0) x = make_double2(f2d_fast(f.x), f2d_fast(f.y));   // x was 0: no add
-                    else { x.x += f2d_fast(f.x); x.y += f2d_fast(f.y); }
-                    xq[q + e] = x;
-                    if (k == 0) x0f[q + e] = f;          // x0 = f exactly when unscaled
-                }
-            }
-            if (k == 0) x0_exact = !scaled && e > -60 && e < 60;   // the FP32-pair residual stays normal
-            __syncthreads();
-        }
-        const bool rnd = check_broken && (ctrl->round_matvec & 2);   // precision probe, Arnoldi solves
-        for (int q = tid; q < cl; q += kInvThreads) {
-            const int p = dir ? (n - 1 - (q0 + q)) : (q0 + q);
-            out[base + p] = conv<TO>(rnd ? round_c64(xq[q]) : xq[q]);
-        }
+    for (int i = 0; i < kSolveFrags; ++i) {
+        a[2 * i] = __ldg(frag + i * 96);
+        a[2 * i + 1] = __ldg(frag + i * 96 + 32);
     }
 }
 
-// Complex64 solve of the mixed path's Krylov basis (one CTA per chunk of a row):
-//   x0 = M b_hi                       FP32
-//   r  = b - U~ x0                    FP32 pairs: U~ = uh + ul, b = bh + bl (bl = 0 for a
-//                                     complex64 operand), error-free products and sums
-//   x  = x0 + M r                     FP32, rounded once
-// The refinement makes the operator seen by the basis U^-1 to ~1e-13 (the FP32 band of
-// M alone perturbs it by ~1e-7, which shifts high eigenvalues systematically).  A
-// double2 operand (the FP64 first vector) is used as hi + lo, a complex64 operand as
-// stored, so the solve acts on exactly the vector kept in the basis.
-template <int KD, bool STAGE, typename TI, typename TV>
-__global__ void __launch_bounds__(kInvThreads) k_solve_mixed(InvTab tab, const TI* __restrict__ in,
-                                                             float2* __restrict__ out, TV* __restrict__ vstore,
-                                                             Ctrl* __restrict__ ctrl, int dir, int scale_mode,
-                                                             int check_broken, float4* __restrict__ v0s,
-                                                             const float4* __restrict__ bpart, int bG) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ __align__(8) unsigned long long s_bar;
-    const int n = tab.n, w = tab.w;
-    const int l = blockIdx.y, tid = threadIdx.x;
-    const int q0 = blockIdx.x * tab.chunk;
-    int cl, R0, RB;
-    inv_region(n, q0, tab.chunk, 1, w, KD, &cl, &R0, &RB);
-    const int R0p = (R0 + 3) & ~3;
-    unsigned char* sp = smem_raw;                  // bulk-copy destinations first (16-byte aligned)
-    float* Ms = reinterpret_cast<float*>(sp);
-    float* Uh = Ms + (size_t)(w + 1) * R0p;
-    float* Ul = Uh + (size_t)(KD + 1) * R0p;
-    if (STAGE) sp += (size_t)(w + 1) * R0p * 4 + (size_t)2 * (KD + 1) * R0p * 4;
-    float2* bh = reinterpret_cast<float2*>(sp);
-    float2* bl = bh + RB;
-    float2* x0 = bl + RB;                          // 16-byte aligned
-    float2* r32 = x0 + ((R0 + 1) & ~1);            // 16-byte aligned; 2 slots of padding
-
-    const float* Mg = tab.m + q0;
-    const float* Uhg = tab.uh + q0;
-    const float* Ulg = tab.ul + q0;
-    if (STAGE) {
-        if (tid == 0) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_bar)) : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-        __syncthreads();
-        if (tid == 0) {
-            const unsigned row = (unsigned)R0p * 4;
-            const unsigned bytes = (unsigned)(w + 1 + 2 * (KD + 1)) * row;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                         :: "r"(smem_u32(&s_bar)), "r"(bytes) : "memory");
-            for (int j = 0; j <= w; ++j) bulk_g2s(Ms + (size_t)j * R0p, Mg + (size_t)j * tab.npad, row, &s_bar);
-            for (int d = 0; d <= KD; ++d) {
-                bulk_g2s(Uh + (size_t)d * R0p, Uhg + (size_t)d * tab.npad, row, &s_bar);
-                bulk_g2s(Ul + (size_t)d * R0p, Ulg + (size_t)d * tab.npad, row, &s_bar);
-            }
-        }
-    }
-    pdl_wait();
-    if (check_broken && ctrl->broken) {
-        if (STAGE) mbar_wait0(&s_bar);
-        return;
-    }
-    const float* mbase = STAGE ? Ms : Mg;
-    const size_t mstride = STAGE ? (size_t)R0p : (size_t)tab.npad;
-    const float* uhb = STAGE ? Uh : Uhg;
-    const float* ulb = STAGE ? Ul : Ulg;
-    const size_t ustride = STAGE ? (size_t)R0p : (size_t)tab.npad;
-    const size_t base = (size_t)l * n;
-    constexpr bool kWide = sizeof(TI) == sizeof(double2);
-    if constexpr (kWide) {
-        // the FP64 first vector (once per step): scaled in FP64, kept as hi + lo
-        const double sc = scale_mode ? ctrl->inv_beta : 1.0;
-        for (int q = tid; q < R0 + w + 2; q += kInvThreads) {
-            float2 hi = make_float2(0.f, 0.f), lo = make_float2(0.f, 0.f);
-            if (q < RB) {
-                const int p = dir ? (n - 1 - (q0 + q)) : (q0 + q);
-                const TI t = in[base + p];
-                double2 b = make_double2((double)t.x, (double)t.y);
-                if (scale_mode) { b.x *= sc; b.y *= sc; }
-                hi = make_float2(d2f_fast(b.x), d2f_fast(b.y));
-                lo = make_float2(d2f_fast(b.x - f2d_fast(hi.x)), d2f_fast(b.y - f2d_fast(hi.y)));
-                if (q < cl) {
-                    if (vstore) vstore[base + p] = conv<TV>(b);
-                    if (v0s) v0s[base + p] = make_float4(hi.x, hi.y, lo.x, lo.y);
-                }
-                bh[q] = hi;
-                bl[q] = lo;
-            }
-            r32[q] = hi;
-        }
-    } else {
-        // a complex64 vector: scaled by 1/beta as an FP32 pair, rounded once (no FP64
-        // instruction per element).  late: 1/beta from the Gram-Schmidt kernel's norm
-        // partials, formed by warp 0 while the other warps load (see k_solve_inv)
-        const bool late = scale_mode && bpart;
-        __shared__ float2 s_ibf;
-        __shared__ int s_brk;
-        if (late && (tid >> 5) == 0) {
-            const double beta = gs_beta<true>(bpart, bG);
-            if ((tid & 31) == 0) {
-                s_brk = gs_record_beta(ctrl, beta, blockIdx.x == 0 && blockIdx.y == 0);
-                const double ib = 1.0 / beta;
-                const float h = (float)ib;
-                s_ibf = make_float2(h, (float)(ib - (double)h));
-            }
-        }
-        float sh = 1.f, sl = 0.f;
-        if (scale_mode && !late) { sh = ctrl->inv_beta_f[0]; sl = ctrl->inv_beta_f[1]; }
-        const int t0 = late ? tid - 32 : tid, tstep = late ? kInvThreads - 32 : kInvThreads;
-        if (t0 >= 0)
-            for (int q = t0; q < R0 + w + 2; q += tstep) {
-                float2 hi = make_float2(0.f, 0.f);
-                if (q < RB) {
-                    const int p = dir ? (n - 1 - (q0 + q)) : (q0 + q);
-                    const TI t = in[base + p];
-                    hi = make_float2((float)t.x, (float)t.y);
-                    if (scale_mode && !late) hi = make_float2(mul_pair(hi.x, sh, sl), mul_pair(hi.y, sh, sl));
-                    if (vstore && q < cl && !late) vstore[base + p] = conv<TV>(hi);
-                    bh[q] = hi;
-                    bl[q] = make_float2(0.f, 0.f);
-                }
-                r32[q] = hi;
-            }
-        if (late) {
-            __syncthreads();
-            if (s_brk) {                               // uniform: the same beta in every CTA
-                if (STAGE) mbar_wait0(&s_bar);
-                return;
-            }
-            sh = s_ibf.x;
-            sl = s_ibf.y;
-            for (int q = tid; q < RB; q += kInvThreads) {
-                const float2 b = bh[q];
-                const float2 hi = make_float2(mul_pair(b.x, sh, sl), mul_pair(b.y, sh, sl));
-                bh[q] = hi;
-                r32[q] = hi;
-                if (vstore && q < cl) vstore[base + (dir ? (n - 1 - (q0 + q)) : (q0 + q))] = conv<TV>(hi);
-            }
-        }
-    }
-    bool ok = true;
-    if (STAGE) ok = mbar_wait0(&s_bar, wait_budget(ctrl, kInvWaitLimit));
-    if (!__syncthreads_and(ok)) {
-        if (tid == 0) ctrl->wait_timeout = 1;
-        if (STAGE) mbar_wait0(&s_bar);             // let copies in flight land before exit
-        return;
-    }
-    for (int q = 2 * tid; q < R0; q += 2 * kInvThreads) {
-        const float4 f = inv_apply2<STAGE>(mbase + q, mstride, r32, q, w);
-        if (q + 1 < R0) *reinterpret_cast<float4*>(x0 + q) = f;
-        else x0[q] = make_float2(f.x, f.y);
-    }
-    __syncthreads();
-    const int Rr = min(n - q0, cl + w);
-    for (int q = tid; q < cl + w; q += kInvThreads) {
-        float2 r = make_float2(0.f, 0.f);
-        if (q < Rr) {
-            float hr = 0.f, lr = 0.f, hi_ = 0.f, li = 0.f;
+// Sixteen outputs of eight planes: o[0], o[1] = planes 2j, 2j+1 (j = lane % 4) of output lane / 4,
+// o[2], o[3] of output lane / 4 + 8.  frag: the block's M fragments (this lane's), a: what load_frags
+// took of them; r: this lane's plane (lane / 4) of the leading parts, as pairs of entries, from the
+// block's first output on + lane % 4; the middle and last parts `part` words further each.
+__device__ __forceinline__ void band_tile(float (&o)[4], const uint4* frag, uint4 (&a)[2 * kSolveFrags], int ks,
+                                          const unsigned* r, int part) {
+    float c1[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f}, c3[4] = {0.f, 0.f, 0.f, 0.f};
+    float c4[4] = {0.f, 0.f, 0.f, 0.f}, c5[4] = {0.f, 0.f, 0.f, 0.f}, c6[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int k0 = 0;;) {
+        uint4 al[kSolveFrags];
 #pragma unroll
-            for (int d = 0; d <= KD; ++d) {
-                if (q + d < n - q0) {
-                    const float uh = uhb[(size_t)d * ustride + q], ul = ulb[(size_t)d * ustride + q];
-                    const float2 xv = x0[q + d];
-                    acc_prod(hr, lr, uh, ul, xv.x);
-                    acc_prod(hi_, li, uh, ul, xv.y);
-                }
-            }
-            const float2 b_h = bh[q], b_l = bl[q];
-            float s, e;
-            two_sum(b_h.x, -hr, s, e);
-            r.x = __fadd_rn(s, __fadd_rn(e, __fsub_rn(b_l.x, lr)));
-            two_sum(b_h.y, -hi_, s, e);
-            r.y = __fadd_rn(s, __fadd_rn(e, __fsub_rn(b_l.y, li)));
+        for (int i = 0; i < kSolveFrags; ++i) al[i] = __ldg(frag + i * 96 + 64);
+#pragma unroll
+        for (int i = 0; i < kSolveFrags; ++i) {
+            const unsigned h0 = r[8 * i], h1 = r[8 * i + 4], m0 = r[8 * i + part], m1 = r[8 * i + 4 + part];
+            const unsigned l0 = r[8 * i + 2 * part], l1 = r[8 * i + 4 + 2 * part];
+            mma_bf16(c1, a[2 * i], h0, h1);
+            mma_bf16(c2, a[2 * i], m0, m1);
+            mma_bf16(c3, a[2 * i + 1], h0, h1);
+            mma_bf16(c4, a[2 * i + 1], m0, m1);
+            mma_bf16(c5, a[2 * i], l0, l1);
+            mma_bf16(c6, al[i], h0, h1);
         }
-        r32[q] = r;
+        k0 += kSolveFrags;
+        if (k0 >= ks) break;
+        r += 8 * kSolveFrags;
+        frag += 96 * kSolveFrags;
+        load_frags(a, frag);
     }
-    __syncthreads();
-    for (int q = 2 * tid; q < cl; q += 2 * kInvThreads) {
-        const float4 d = inv_apply2<STAGE>(mbase + q, mstride, r32, q, w);
-        float2 x = x0[q];
-        out[base + (dir ? (n - 1 - (q0 + q)) : (q0 + q))] = make_float2(__fadd_rn(x.x, d.x), __fadd_rn(x.y, d.y));
-        if (q + 1 < cl) {
-            x = x0[q + 1];
-            out[base + (dir ? (n - 2 - (q0 + q)) : (q0 + q + 1))] = make_float2(__fadd_rn(x.x, d.z), __fadd_rn(x.y, d.w));
-        }
-    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = c1[j] + ((c2[j] + c3[j]) + (c4[j] + (c5[j] + c6[j])));
 }
 
-template <int KD, bool STAGE>
-static cudaError_t solve_mixed_launch(const InvTab& tab, int nrows, const void* in, int in_prec, void* out,
-                                      int out_prec, void* vstore, int v_prec, Ctrl* ctrl, int dir, int scale_mode,
-                                      int check_broken, cudaStream_t s, float4* v0s, const void* bpart, int bG) {
-    if (out_prec != 1) return cudaErrorInvalidValue;
-    size_t smem = 0;
-    for (int c = 0; c < tab.nchunks; ++c)
-        smem = std::max(smem, inv_smem_bytes_mixed(tab.n, c * tab.chunk, tab.chunk, tab.w, KD, STAGE));
-    dim3 grid(tab.nchunks, nrows), block(kInvThreads);
-#define GB_MIX_CASE(TI_, TV_)                                                                                    \
-    {                                                                                                            \
-        auto kern = k_solve_mixed<KD, STAGE, TI_, TV_>;                                                          \
-        if (smem > 48 * 1024) {                                                                                  \
-            cudaError_t ea = allow_max_smem(kern);                                                               \
-            if (ea != cudaSuccess) return ea;                                                                    \
-        }                                                                                                        \
-        cudaError_t el = launch_pdl(kern, grid, block, smem, s, tab, (const TI_*)in, (float2*)out, (TV_*)vstore,  \
-                                    ctrl, dir, scale_mode, check_broken, v0s, (const float4*)bpart, bG);         \
-        return el != cudaSuccess ? el : cudaGetLastError();                                                      \
-    }
-    // in: the FP64 first vector (with its FP64 copy stored) or a complex64 vector
-    if (in_prec == 0 && v_prec == 0) GB_MIX_CASE(double2, double2)
-    if (v0s) return cudaErrorInvalidValue;
-    if (in_prec == 1) GB_MIX_CASE(float2, float2)
-#undef GB_MIX_CASE
-    return cudaErrorInvalidValue;
+// a plane's entry as its three bfloat16 parts (v = h + m + l exactly), `part` halves apart
+__device__ __forceinline__ void put_split(unsigned short* r, int part, float v) {
+    const unsigned h = __float_as_uint(v) & 0xffff0000u;
+    const float v1 = __fsub_rn(v, __uint_as_float(h));
+    const unsigned m = __float_as_uint(v1) & 0xffff0000u;
+    const float v2 = __fsub_rn(v1, __uint_as_float(m));
+    r[0] = (unsigned short)(h >> 16);
+    r[part] = (unsigned short)(m >> 16);
+    r[2 * part] = (unsigned short)(__float_as_uint(v2) >> 16);
 }
 
 template <int KD, bool R64, bool STAGE>
-static cudaError_t solve_inv_launch(const InvTab& tab, int nrows, const void* in, int in_prec, void* out,
-                                    int out_prec, void* vstore, int v_prec, Ctrl* ctrl, int dir,
-                                    int scale_mode, int check_broken, cudaStream_t s, const void* bpart, int bG) {
-    const int P = R64 ? tab.refine : 0;
-    size_t smem = 0;
-    for (int c = 0; c < tab.nchunks; ++c)
-        smem = std::max(smem, inv_smem_bytes(tab.n, c * tab.chunk, tab.chunk, P, tab.w, KD, STAGE, R64));
-    dim3 grid(tab.nchunks, nrows), block(kInvThreads);
-#define GB_INV_CASE(TI_, TO_, TV_)                                                                               \
-    {                                                                                                            \
-        auto kern = k_solve_inv<KD, R64, STAGE, TI_, TO_, TV_>;                                                  \
-        if (smem > 48 * 1024) {                                                                                  \
-            cudaError_t ea = allow_max_smem(kern);                                                               \
-            if (ea != cudaSuccess) return ea;                                                                    \
-        }                                                                                                        \
-        cudaError_t el = launch_pdl(kern, grid, block, smem, s, tab, (const TI_*)in, (TO_*)out, (TV_*)vstore,     \
-                                    ctrl, dir, scale_mode, check_broken, (const double*)bpart, bG);              \
-        return el != cudaSuccess ? el : cudaGetLastError();                                                      \
+__global__ void __launch_bounds__(kRowBlock) k_solve_rows(InvTab tab, int nl, const void* in, int in_prec, void* out,
+                                                          int out_prec, void* vstore, float4* v0s, Ctrl* ctrl, int dir,
+                                                          int scale_mode, int check_broken, const void* bpart, int bG) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned s_red[kRowWarps];
+    __shared__ double s_ib;                            // 1/beta (FP64 solve)
+    __shared__ float2 s_ibf;                           // 1/beta as an FP32 pair (complex64 solve)
+    __shared__ int s_brk, s_skip;
+    constexpr int UP = inv_upitch(KD);                 // entries of a row of U~'s tables
+    const int n = tab.n, w = tab.w, P = R64 ? tab.refine : 1, ks = tab.ks;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = (int)(blockDim.x >> 5) - 1;
+    const int q0 = blockIdx.x * tab.chunk, left = n - q0;
+    const int lg = tab.lg, rmask = (1 << lg) - 1, l0 = blockIdx.y << lg;
+    const int rows = min(1 << lg, nl - l0);
+    const int lnt = max(lg - 2, 0);                    // log2 of the plane groups of a tile column
+    int cl, R0, RB;
+    inv_region(n, q0, tab.chunk, P, w, KD, &cl, &R0, &RB);
+    const int PL = tab.pl;                             // from a plane's leading part to its next
+    const int PQ = tab.pq, PX = tab.px, PD = tab.pd, PB = tab.pb;
+    const InvLayout& ly = tab.ly;
+    const double* const Us = reinterpret_cast<const double*>(smem_raw + ly.u);
+    const float2* const Ufs = reinterpret_cast<const float2*>(smem_raw + ly.uf);
+    double2* const bq = reinterpret_cast<double2*>(smem_raw + ly.b);      // R64: right-hand side [row][q]
+    float4* const bf = reinterpret_cast<float4*>(smem_raw + ly.b);        // complex64: FP32 pairs [row][q]
+    double2* const xd = reinterpret_cast<double2*>(smem_raw + ly.x);      // R64: iterate [row][q]
+    unsigned short* const r16 = reinterpret_cast<unsigned short*>(smem_raw + ly.r16);   // residual planes
+    float2* const x0f = reinterpret_cast<float2*>(smem_raw + ly.x0);      // first iterate [row][q]
+    const uint4* const Mg = reinterpret_cast<const uint4*>(tab.mf) + (size_t)(q0 >> 4) * ks * 96 + lane;
+    const bool late = scale_mode && bpart;             // beta comes from norm partials
+
+    if (warp == nw) {
+        // this warp forms 1/beta
+        pdl_wait();
+        const bool writer = blockIdx.x == 0 && blockIdx.y == 0 && !(check_broken == 1 && ctrl->broken);
+        if constexpr (R64) {
+            if (late) {
+                const double beta = gs_beta(bpart, bG);
+                if (lane == 0) {
+                    s_brk = gs_record_beta(ctrl, beta, writer);
+                    s_ib = 1.0 / beta;
+                }
+            }
+            __syncthreads();
+        } else if (late) {
+            const float2 t = gs_norm2_pair(reinterpret_cast<const float4*>(bpart), bG);
+            if (lane == 0) {
+                s_brk = t.x < (float)DBL_EPSILON || (t.x == (float)DBL_EPSILON && t.y < 0.f);
+                s_ibf = inv_sqrt_pair(t.x, t.y);
+            }
+            __syncthreads();
+            if (lane == 0 && writer) gs_record_beta(ctrl, sqrt((double)t.x + (double)t.y), true);
+        }
+        return;
     }
-    // combinations the runtime uses: refined solves store double2 (or nothing)
-    const int key = in_prec * 4 + out_prec * 2 + v_prec;
-    switch (key) {
-        case 0: GB_INV_CASE(double2, double2, double2)
-        case 2: GB_INV_CASE(double2, float2, double2)
-        case 4: GB_INV_CASE(float2, double2, double2)
-        case 6: GB_INV_CASE(float2, float2, double2)
-        default: return cudaErrorInvalidValue;
+    // ---- workers.  The first tile's M fragments are on their way before the wait; everything
+    // below reads what earlier kernels wrote.
+    uint4 fr[2 * kSolveFrags];
+    const int ft = warp >> lnt;                        // the warp's first block of outputs
+    if (16 * ft < R0) {
+        load_frags(fr, Mg + ft * ks * 96);
+#pragma unroll
+        for (int i = 0; i < kSolveFrags; ++i) prefetch_l1(Mg + ft * ks * 96 + i * 96 + 64);
     }
-#undef GB_INV_CASE
+    if (STAGE) {
+        // U~'s slices: contiguous rows of R0p entries (sizes and addresses multiples of 16 bytes)
+        const int nc = ((R0 + 3) & ~3) * UP / 2;
+        const double2* gf = reinterpret_cast<const double2*>(tab.uf + (size_t)q0 * UP);
+        const double2* gu = reinterpret_cast<const double2*>(tab.u + (size_t)q0 * UP);
+        for (int i = tid; i < nc; i += (32 * nw)) {
+            cp_async16(smem_raw + ly.uf + 16 * i, gf + i);
+            if (R64) cp_async16(smem_raw + ly.u + 16 * i, gu + i);
+        }
+    }
+    pdl_wait();
+    const int gdir = dir ? -1 : 1;
+    const size_t gbase = (size_t)l0 * n + (dir ? n - 1 - q0 : q0);
+    auto gidx = [&](int row, int q) { return gbase + (long)(row * n + gdir * q); };
+    // 1: after a happy breakdown, 2: a step of this call gave up on a wait -- nothing is written.  One
+    // read for the CTA: this launch's first CTA may set ctrl->broken while others start
+    int skip = 0;
+    if (tid == 0)
+        skip = check_broken == 1   ? *(volatile const int*)&ctrl->broken
+               : check_broken == 2 ? *(volatile const int*)&ctrl->wait_timeout
+                                   : 0;
+    // zeros past the chunk's data: the residual past the right-hand side (a tile reads 16 ks entries
+    // from its first output on; planes without a row are zero), the iterates past the last element
+    auto zero_tails = [&]() {
+        if (tid == 0) s_skip = skip;
+        for (int g = warp; g < max(2 << lg, 8); g += nw) {
+            const int t0 = g < 2 * rows ? RB : 0;
+            unsigned short* rr = r16 + g * PQ;
+            if ((t0 & 1) && lane < 3) rr[lane * PL + t0] = 0;
+            for (int i = ((t0 + 1) >> 1) + lane; i < (PQ >> 1); i += 32) {
+                reinterpret_cast<unsigned*>(rr)[i] = 0;
+                reinterpret_cast<unsigned*>(rr + PL)[i] = 0;
+                reinterpret_cast<unsigned*>(rr + 2 * PL)[i] = 0;
+            }
+        }
+        if (warp >= nw / 2) {
+            const int xde = (min(left, cl + (P >= 2 ? P - 1 : 1) * (w + KD)) + 15) & ~15;
+            for (int row = warp - nw / 2; row < rows; row += nw / 2) {
+                for (int q = ((R0 + 15) & ~15) + lane; q < PX; q += 32) x0f[row * PX + q] = make_float2(0.f, 0.f);
+                if (R64)
+                    for (int q = xde + lane; q < PD; q += 32) xd[row * PD + q] = make_double2(0.0, 0.0);
+            }
+        }
+    };
+    const int probe = R64 && check_broken == 1 ? ctrl->round_matvec : 0;
+
+    // right-hand side: a warp takes 32-element segments of the rows, kPre of them loaded at once
+    constexpr int kPre = 3;
+    const int nbs = ((RB + 31) >> 5) << lg;
+    double fin = 1.0;                                  // R64: factor of x and v at the end, if `scaled`
+    bool scaled = scale_mode != 0;
+    if constexpr (R64) {
+        if (scale_mode && !late) fin = ctrl->inv_beta;
+        auto keep = [&](int it, double2 b) {
+            const int row = it & rmask, q = (it >> lg) * 32 + lane;
+            if (row < rows && q < RB) {
+                bq[row * PB + q] = b;
+                unsigned short* rr = r16 + 2 * row * PQ + q;
+                put_split(rr, PL, d2f_fast(b.x));
+                put_split(rr + PQ, PL, d2f_fast(b.y));
+            }
+        };
+        unsigned hmax = 0;
+        for (int i0 = warp;;) {
+            double2 pre[kPre];
+#pragma unroll
+            for (int u = 0; u < kPre; ++u) {
+                const int it = i0 + u * nw, row = it & rmask, q = (it >> lg) * 32 + lane;
+                pre[u] = make_double2(0.0, 0.0);
+                if (row < rows && q < RB) {
+                    if (in_prec == 0) pre[u] = reinterpret_cast<const double2*>(in)[gidx(row, q)];
+                    else {
+                        const float2 t = reinterpret_cast<const float2*>(in)[gidx(row, q)];
+                        pre[u] = make_double2(f2d_fast(t.x), f2d_fast(t.y));
+                    }
+                }
+            }
+            if (i0 == warp) zero_tails();              // while the first loads are in flight
+#pragma unroll
+            for (int u = 0; u < kPre; ++u) {
+                keep(i0 + u * nw, pre[u]);
+                hmax = max(hmax, max((unsigned)__double2hiint(pre[u].x) & 0x7fffffffu,
+                                     (unsigned)__double2hiint(pre[u].y) & 0x7fffffffu));
+            }
+            i0 += kPre * nw;
+            if (i0 >= nbs) break;
+        }
+        hmax = __reduce_max_sync(0xffffffffu, hmax);
+        if (lane == 0) s_red[warp] = hmax;
+        if (STAGE) cp_async_wait_all();
+        worker_sync(nw);
+        hmax = __reduce_max_sync(0xffffffffu, s_red[lane & (nw - 1)]);
+        // a right-hand side whose largest exponent leaves the range where the FP32 residuals
+        // (down to 2^-50 of it) stay normal is scaled by a power of two, and x back at the end
+        const int e = (int)(hmax >> 20) - 1022;
+        if (hmax != 0 && hmax < 0x7ff00000u && (e < -60 || e > 60)) {
+            scaled = true;
+            fin = fin * pow2_double(e / 2) * pow2_double(e - e / 2);
+            for (int it = warp; it < nbs; it += nw) {
+                const int row = it & rmask, q = (it >> lg) * 32 + lane;
+                if (row >= rows || q >= RB) continue;
+                const double2 b = bq[row * PB + q];
+                keep(it, make_double2(scale_pow2(b.x, -e), scale_pow2(b.y, -e)));
+            }
+            worker_sync(nw);
+        }
+    } else {
+        if (in_prec == 0) {
+            // the FP64 first vector (once per step): scaled in FP64, kept as hi + lo
+            zero_tails();
+            const double sc = scale_mode ? ctrl->inv_beta : 1.0;
+            for (int it = warp; it < nbs; it += nw) {
+                const int row = it & rmask, q = (it >> lg) * 32 + lane;
+                if (row >= rows || q >= RB) continue;
+                const size_t gi = gidx(row, q);
+                double2 b = reinterpret_cast<const double2*>(in)[gi];
+                if (scale_mode) { b.x *= sc; b.y *= sc; }
+                const float2 hi = make_float2(d2f_fast(b.x), d2f_fast(b.y));
+                const float2 lo = make_float2(d2f_fast(b.x - f2d_fast(hi.x)), d2f_fast(b.y - f2d_fast(hi.y)));
+                if (q < cl) {
+                    if (vstore) reinterpret_cast<double2*>(vstore)[gi] = b;
+                    if (v0s) v0s[gi] = make_float4(hi.x, hi.y, lo.x, lo.y);
+                }
+                unsigned short* rr = r16 + 2 * row * PQ + q;
+                put_split(rr, PL, hi.x);
+                put_split(rr + PQ, PL, hi.y);
+                bf[row * PB + q] = make_float4(hi.x, hi.y, lo.x, lo.y);
+            }
+        } else {
+            // a complex64 vector: scaled by 1/beta as an FP32 pair, rounded once
+            const float2* src = reinterpret_cast<const float2*>(in);
+            float sh = 1.f, sl = 0.f;
+            int brk = 0;
+            for (int i0 = warp;;) {
+                float2 pre[kPre];
+#pragma unroll
+                for (int u = 0; u < kPre; ++u) {
+                    const int it = i0 + u * nw, row = it & rmask, q = (it >> lg) * 32 + lane;
+                    pre[u] = row < rows && q < RB ? src[gidx(row, q)] : make_float2(0.f, 0.f);
+                }
+                if (i0 == warp) {
+                    zero_tails();                      // while the first loads are in flight
+                    if (late) {
+                        __syncthreads();               // with the warp that forms 1/beta
+                        sh = s_ibf.x;
+                        sl = s_ibf.y;
+                        brk = s_brk;
+                    } else if (scale_mode) {
+                        sh = ctrl->inv_beta_f[0];
+                        sl = ctrl->inv_beta_f[1];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kPre; ++u) {
+                    const int it = i0 + u * nw, row = it & rmask, q = (it >> lg) * 32 + lane;
+                    if (row >= rows || q >= RB) continue;
+                    float2 v = pre[u];
+                    if (scale_mode) v = make_float2(mul_pair(v.x, sh, sl), mul_pair(v.y, sh, sl));
+                    if (vstore && q < cl && !brk) reinterpret_cast<float2*>(vstore)[gidx(row, q)] = v;
+                    unsigned short* rr = r16 + 2 * row * PQ + q;
+                    put_split(rr, PL, v.x);
+                    put_split(rr + PQ, PL, v.y);
+                    bf[row * PB + q] = make_float4(v.x, v.y, 0.f, 0.f);
+                }
+                i0 += kPre * nw;
+                if (i0 >= nbs) break;
+            }
+        }
+        if (STAGE) cp_async_wait_all();
+        worker_sync(nw);
+        if (late && s_brk) return;                     // uniform: the same beta in every CTA
+    }
+    if (s_skip) {
+        if (R64) __syncthreads();
+        return;
+    }
+
+    const bool pair = !R64 || P >= 2;                  // the first residual comes from FP32 pairs
+    const double* const ub = STAGE ? Us : tab.u + (size_t)q0 * UP;
+    const float2* const ufb = STAGE ? Ufs : tab.uf + (size_t)q0 * UP;
+    for (int k = 0; k <= P; ++k) {
+        const int Rk = min(left, cl + (P - k) * (w + KD));
+        if (k > 0) {
+            if (16 * ft < Rk) load_frags(fr, Mg + ft * ks * 96);
+            const int Rr = min(left, Rk + w), nrs = ((Rr + 31) >> 5) << lg;
+            for (int it = warp; it < nrs; it += nw) {
+                const int row = it & rmask, q = (it >> lg) * 32 + lane;
+                if (row >= rows || q >= Rr) continue;
+                unsigned short* rr = r16 + 2 * row * PQ + q;
+                if (k == 1 && pair) {
+                    // r = b - U~ x0, x0 exact in FP32, from FP32 pairs: relative error ~2^-48 |b| / |r|,
+                    // far below what a pass needs whose result is refined again or rounded to FP32
+                    const float2* xp = x0f + row * PX + q;
+                    const float2* up = ufb + q * UP;
+                    float4 b;                          // b's FP32 pairs
+                    if constexpr (R64) {
+                        const double2 v = bq[row * PB + q];
+                        b = make_float4(d2f_fast(v.x), d2f_fast(v.y), d2f_low(v.x), d2f_low(v.y));
+                    } else {
+                        b = bf[row * PB + q];
+                    }
+                    float hr = 0.f, lr = 0.f, hi = 0.f, li = 0.f;
+#pragma unroll
+                    for (int d = 0; d <= KD; ++d) {
+                        const float2 u = row_ld<STAGE>(up + d);
+                        const float2 xv = xp[d];
+                        acc_prod(hr, lr, u.x, u.y, xv.x);
+                        acc_prod(hi, li, u.x, u.y, xv.y);
+                    }
+                    float s, e;
+                    two_sum(b.x, -hr, s, e);
+                    put_split(rr, PL, __fadd_rn(s, __fadd_rn(e, __fsub_rn(b.z, lr))));
+                    two_sum(b.y, -hi, s, e);
+                    put_split(rr + PQ, PL, __fadd_rn(s, __fadd_rn(e, __fsub_rn(b.w, li))));
+                } else if constexpr (R64) {
+                    const double2* xp = xd + row * PD + q;
+                    const double* up = ub + q * UP;
+                    double2 r = bq[row * PB + q];
+#pragma unroll
+                    for (int d = 0; d <= KD; ++d) {
+                        const double u = row_ld<STAGE>(up + d);
+                        const double2 xv = xp[d];
+                        r.x = fma(-u, xv.x, r.x);
+                        r.y = fma(-u, xv.y, r.y);
+                    }
+                    put_split(rr, PL, d2f_fast(r.x));
+                    put_split(rr + PQ, PL, d2f_fast(r.y));
+                }
+            }
+            if (R64 && k == P) __syncthreads();        // with the warp that forms 1/beta
+            else worker_sync(nw);
+        }
+        const bool last = k == P;
+        if (R64 && last && late) {
+            if (s_brk) return;                         // uniform: the same beta in every CTA
+            fin *= s_ib;
+        }
+        const bool rnd = R64 && (probe & 2);           // precision probe
+        const int nt = (warp & ((1 << lnt) - 1)), row = 4 * nt + (lane & 3);
+        const unsigned* rt = reinterpret_cast<const unsigned*>(r16) + (8 * nt + (lane >> 2)) * (PQ >> 1) + (lane & 3);
+        for (int bk = ft; 16 * bk < Rk; bk += nw >> lnt) {
+            const uint4* frag = Mg + bk * ks * 96;
+            if (bk != ft) load_frags(fr, frag);
+            float d[4];
+            band_tile(d, frag, fr, ks, rt + 8 * bk, PL >> 1);
+            if (row >= rows) continue;
+            const int q = 16 * bk + (lane >> 2);
+            if (k == 0 && pair) {
+                float2* xp = x0f + row * PX + q;
+                xp[0] = make_float2(d[0], d[1]);
+                xp[8] = make_float2(d[2], d[3]);
+            } else if constexpr (R64) {
+                double2 x[2];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) x[j] = make_double2(f2d_fast(d[2 * j]), f2d_fast(d[2 * j + 1]));
+                double2* xp = xd + row * PD + q;
+                if (k == 1 && pair) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const float2 x0 = x0f[row * PX + q + 8 * j];
+                        x[j].x += f2d_fast(x0.x);
+                        x[j].y += f2d_fast(x0.y);
+                    }
+                } else if (k > 0) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const double2 xo = xp[8 * j];
+                        x[j].x += xo.x;
+                        x[j].y += xo.y;
+                    }
+                }
+                if (!last) {
+                    xp[0] = x[0];
+                    xp[8] = x[1];
+                    continue;
+                }
+                if (scaled) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) x[j] = make_double2(x[j].x * fin, x[j].y * fin);
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (q + 8 * j >= cl) break;
+                    const size_t gi = gidx(row, q + 8 * j);
+                    // (the integer conversions: an FP64 conversion instruction costs what an FMA does)
+                    const float2 f = make_float2(d2f_fast(x[j].x), d2f_fast(x[j].y));
+                    if (out_prec) reinterpret_cast<float2*>(out)[gi] = f;
+                    else reinterpret_cast<double2*>(out)[gi] = rnd ? make_double2(f2d_fast(f.x), f2d_fast(f.y)) : x[j];
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (q + 8 * j >= cl) break;
+                    const float2 x0 = x0f[row * PX + q + 8 * j];
+                    reinterpret_cast<float2*>(out)[gidx(row, q + 8 * j)] =
+                        make_float2(__fadd_rn(x0.x, d[2 * j]), __fadd_rn(x0.y, d[2 * j + 1]));
+                }
+            }
+        }
+        if (R64 && last && vstore) {
+            // the basis vector v = in / beta (fin also undoes a power-of-two scaling of b)
+            const int nvs = ((cl + 31) >> 5) << lg;
+            for (int it = warp; it < nvs; it += nw) {
+                const int row = it & rmask, q = (it >> lg) * 32 + lane;
+                if (row >= rows || q >= cl) continue;
+                const double2 b = bq[row * PB + q];
+                reinterpret_cast<double2*>(vstore)[gidx(row, q)] = make_double2(b.x * fin, b.y * fin);
+            }
+        }
+        if (!last) worker_sync(nw);
+    }
+}
+
+template <int KD, bool R64, bool STAGE>
+static cudaError_t solve_rows_launch(const InvTab& tab, int nl, const void* in, int in_prec, void* out, int out_prec,
+                                     void* vstore, Ctrl* ctrl, int dir, int scale_mode, int check_broken,
+                                     cudaStream_t s, float4* v0s, const void* bpart, int bG) {
+    const size_t smem = tab.ly.bytes;
+    auto kern = k_solve_rows<KD, R64, STAGE>;
+    if (smem > 48 * 1024) {
+        cudaError_t ea = allow_max_smem(kern);
+        if (ea != cudaSuccess) return ea;
+    }
+    dim3 grid(tab.nchunks, (nl + (1 << tab.lg) - 1) >> tab.lg), block(32 * tab.warps + 32);
+    cudaError_t el = launch_pdl(kern, grid, block, smem, s, tab, nl, in, in_prec, out, out_prec, vstore, v0s, ctrl,
+                                dir, scale_mode, check_broken, bpart, bG);
+    return el != cudaSuccess ? el : cudaGetLastError();
 }
 
 template <int KD>
-static cudaError_t solve_inv_kd(const InvTab& tab, int nrows, int refine64, const void* in, int in_prec, void* out,
-                                int out_prec, void* vstore, int v_prec, Ctrl* ctrl, int dir, int scale_mode,
-                                int check_broken, cudaStream_t s, float4* v0s, const void* bpart, int bG) {
+static cudaError_t solve_rows_kd(const InvTab& tab, int nl, int refine64, const void* in, int in_prec, void* out,
+                                 int out_prec, void* vstore, Ctrl* ctrl, int dir, int scale_mode, int check_broken,
+                                 cudaStream_t s, float4* v0s, const void* bpart, int bG) {
+#define GB_ROWS(R64_, STAGE_)                                                                                       \
+    return solve_rows_launch<KD, R64_, STAGE_>(tab, nl, in, in_prec, out, out_prec, vstore, ctrl, dir, scale_mode, \
+                                               check_broken, s, v0s, bpart, bG)
     if (refine64) {
-        if (tab.stage)
-            return solve_inv_launch<KD, true, true>(tab, nrows, in, in_prec, out, out_prec, vstore, v_prec, ctrl, dir,
-                                                    scale_mode, check_broken, s, bpart, bG);
-        return solve_inv_launch<KD, true, false>(tab, nrows, in, in_prec, out, out_prec, vstore, v_prec, ctrl, dir,
-                                                 scale_mode, check_broken, s, bpart, bG);
+        if (tab.stage) GB_ROWS(true, true);
+        GB_ROWS(true, false);
     }
-    if (tab.stage)
-        return solve_mixed_launch<KD, true>(tab, nrows, in, in_prec, out, out_prec, vstore, v_prec, ctrl, dir,
-                                            scale_mode, check_broken, s, v0s, bpart, bG);
-    return solve_mixed_launch<KD, false>(tab, nrows, in, in_prec, out, out_prec, vstore, v_prec, ctrl, dir,
-                                         scale_mode, check_broken, s, v0s, bpart, bG);
+    if (tab.stage) GB_ROWS(false, true);
+    GB_ROWS(false, false);
+#undef GB_ROWS
 }
 
 cudaError_t launch_solve_inv(const InvTab& tab, int nrows, int refine64, const void* in, int in_prec, void* out,
                              int out_prec, void* vstore, int v_prec, Ctrl* ctrl, int dir, int scale_mode,
                              int check_broken, cudaStream_t s, float4* v0s, const void* bpart, int bG) {
     count_launch();
+    // the combinations the runtime uses: FP64-accurate solves store v in FP64 (or not at all), the
+    // complex64 solve gives complex64 and stores v as it came (the split only of an FP64 vector)
+    if (refine64 ? (vstore && v_prec != 0) || v0s : out_prec != 1 || (vstore && v_prec != in_prec) || (v0s && in_prec) || (bpart && !in_prec))
+        return cudaErrorInvalidValue;
     switch (tab.kd) {
 #define GB_KD(K)                                                                                                 \
     case K:                                                                                                      \
-        return solve_inv_kd<K>(tab, nrows, refine64, in, in_prec, out, out_prec, vstore, v_prec, ctrl, dir,      \
-                               scale_mode, check_broken, s, v0s, bpart, bG);
+        return solve_rows_kd<K>(tab, nrows, refine64, in, in_prec, out, out_prec, vstore, ctrl, dir, scale_mode, \
+                                check_broken, s, v0s, bpart, bG);
         GB_KD(1) GB_KD(2) GB_KD(3) GB_KD(4) GB_KD(5) GB_KD(6) GB_KD(7) GB_KD(8)
 #undef GB_KD
         default: return cudaErrorInvalidValue;
