@@ -72,6 +72,9 @@ template <typename T> struct DevTables {
 
 }  // namespace
 
+struct gbprop_batch_ctx;
+static void batch_forget(gbprop_batch_ctx* b, struct gbprop_ctx* h);
+
 struct gbprop_ctx {
     int nl = 0, nr = 0, prec = 0, m = 0, expm_method = 0, double_orth = 0;
     int nfuncs = 1;                   // distinct time functions (values per schedule step)
@@ -128,6 +131,7 @@ struct gbprop_ctx {
     int band_variant = 1;             // tile shape of the band kernel (autotuner)
     int expm_max_cluster = 16;        // 1 inside a large batch
     bool in_batch = false;
+    std::vector<gbprop_batch_ctx*> batches;   // it is a member of
     bool inv_ok = false;              // solves run through the banded approximate inverse
     InvTab inv[2] = {};               // the Krylov-precision solves: [0]: U^-1, [1]: U^-T
     InvTab sinv[2] = {};              // the FP64-accurate solves of the state (same tables, own chunking)
@@ -943,6 +947,7 @@ gbprop_status gbprop_create(gbprop_handle* out, int nl, int nr, int precision, i
 
 gbprop_status gbprop_destroy(gbprop_handle h) {
     if (!h) return GBPROP_OK;
+    for (gbprop_batch_ctx* b : h->batches) batch_forget(b, h);
     if (h->stream) cudaStreamSynchronize(h->stream);
     delete h;
     return GBPROP_OK;
@@ -1830,6 +1835,13 @@ struct gbprop_batch_ctx {
     }
 };
 
+// A member destroyed before its batch (a garbage collector frees a cycle in any order): the batch
+// finishes its work, keeps no pointer to it and can only be destroyed.
+static void batch_forget(gbprop_batch_ctx* b, gbprop_ctx* h) {
+    if (b->stream) cudaStreamSynchronize(b->stream);
+    std::replace(b->hs.begin(), b->hs.end(), h, (gbprop_ctx*)nullptr);
+}
+
 namespace {
 
 // Capture one parallel branch per problem (forked from and joined into the batch stream).
@@ -1882,8 +1894,10 @@ gbprop_status batch_errors(gbprop_batch b, bool block) {
     const int p = b->h_flags[3] - 1;
     if (p < 0 || p >= (int)b->hs.size()) return GBPROP_OK;
     gbprop_ctx* h = b->hs[p];
+    if (!h) return GBPROP_OK;
     // clear every member's flags (only members with a failure have any set)
-    for (gbprop_ctx* x : b->hs) GB_CUDA(cudaMemsetAsync(&x->d_ctrl->lu_info, 0, 3 * sizeof(int), b->stream));
+    for (gbprop_ctx* x : b->hs)
+        if (x) GB_CUDA(cudaMemsetAsync(&x->d_ctrl->lu_info, 0, 3 * sizeof(int), b->stream));
     cudaStream_t keep = h->stream;
     h->stream = b->stream;
     gbprop_status st = report_flags(h, b->h_flags[0], b->h_flags[1], b->h_flags[2]);
@@ -1985,6 +1999,7 @@ gbprop_status gbprop_batch_create(gbprop_batch* out, const gbprop_handle* proble
             }
         }
     }
+    for (gbprop_ctx* h : b->hs) h->batches.push_back(b);
     *out = b;
     return GBPROP_OK;
 }
@@ -1998,6 +2013,8 @@ gbprop_status gbprop_batch_advance(gbprop_batch b, void* const* psi, int nsteps,
     const size_t P = b->hs.size();
     for (size_t p = 0; p < P; ++p)
         if (!psi[p]) return fail(GBPROP_EINVAL, "null wavefunction in batch");
+    for (gbprop_ctx* h : b->hs)
+        if (!h) return fail(GBPROP_EINVAL, "a problem of the batch has been destroyed");
     if (gbprop_status st = batch_errors(b, false)) return st;
     // problem p's nsteps x nfuncs block of the packed scalings
     std::vector<size_t> off(P + 1, 0);
@@ -2073,6 +2090,8 @@ gbprop_status gbprop_batch_destroy(gbprop_batch b) {
     if (!b) return GBPROP_OK;
     if (b->stream) cudaStreamSynchronize(b->stream);
     for (gbprop_handle h : b->hs) {
+        if (!h) continue;
+        h->batches.erase(std::remove(h->batches.begin(), h->batches.end(), b), h->batches.end());
         h->expm_max_cluster = 16;
         h->in_batch = false;
         if (h->inv_ok) set_inv_chunks(h, 0);

@@ -93,3 +93,25 @@ def test_batch_long_radial_grid(precision):
         want, _ = _oracle(p).advance(psi0[i], p.m, p.dt, bp.scalings(i, 2))
         err = rel(bp.psi[i].cpu().numpy().astype(np.complex128), want)
         assert err < (1e-12 if precision == "fp64" else 1e-5), (i, err)
+
+
+@pytest.mark.parametrize("destroyed", [0, 1])
+def test_member_destroyed_before_its_batch(destroyed):
+    """A garbage collector may free the handles of a dropped batch first: the batch refuses to advance and goes
+    without touching them."""
+    import torch
+    from pyprop_gb300 import _native
+    from pyprop_gb300.batch import BatchPropagator, HydrogenProblem
+    bp = BatchPropagator([HydrogenProblem(lmax=2, nr=30, rmax=20.0, m=6, seed=s) for s in (1, 2)], autotune=False)
+    bp.advance(1)
+    bp.handles[destroyed].__del__()
+    with pytest.raises(_native.GbpropError) as e:
+        bp.advance(1)
+    assert "destroyed" in str(e.value)
+    bp.synchronize()
+    bp.batch.__del__()
+    other = bp.handles[1 - destroyed]
+    psi = torch.as_tensor(bp.problems[1 - destroyed].initial_state()).cuda()
+    other.advance(psi, np.zeros(1), 0.01)
+    other.synchronize()
+    assert bool(torch.isfinite(psi.real).all())
