@@ -109,6 +109,7 @@ struct gbprop_ctx {
     float4* d_v0s = nullptr;          // N, the same split into FP32 pairs (re_hi, im_hi, re_lo, im_lo)
     int cgs_grid = 0;                 // > 0: Gram-Schmidt as one cooperative kernel of this many CTAs
     int cgs_cache = 0;                // its V chunk cached in shared memory
+    int cgs_dgrid = 0;                // > 0: the FP64 form with re-orthogonalisation (cgs_cache too)
     int cgs_part_grid = 0;            // the grid d_cgs_part is sized for
     double* d_cgs_part = nullptr;     // its partial sums
     unsigned* d_gridbar = nullptr;    // its grid-barrier words
@@ -739,7 +740,8 @@ gbprop_status enqueue_arnoldi(gbprop_ctx* h, int dorth, double brk_tol) {
     // the FP32-pair split of a complex64 basis's FP64 first vector, written by the inverse-band
     // solve of that vector: read by both Gram-Schmidt forms instead of the FP64 copy
     float4* v0s = (h->d_v0s && h->inv_ok) ? (float4*)h->d_v0s : nullptr;
-    if (fused) GB_CUDA(cudaMemsetAsync(h->d_gridbar, 0, 2 * sizeof(unsigned), s));
+    const bool fused_dorth = h->cgs_dgrid > 0 && dorth && kp == 0;
+    if (fused || fused_dorth) GB_CUDA(cudaMemsetAsync(h->d_gridbar, 0, 2 * sizeof(unsigned), s));
     // beta0 = ||x||
     GB_LAUNCH(launch_norm(0, h->d_x, N, h->d_partials, h->d_counter, h->d_ctrl, s));
     tick(h, GBPROP_PHASE_GRAM_SCHMIDT);
@@ -766,7 +768,13 @@ gbprop_status enqueue_arnoldi(gbprop_ctx* h, int dorth, double brk_tol) {
         // classical Gram-Schmidt against v_0..v_J
         if (fused) {
             GB_LAUNCH(launch_arnoldi_cgs(kp, V, h->d_v0s, N, J, m, h->d_r, h->d_cgs_part, h->d_gridbar, h->d_ctrl,
-                                         h->d_H, J < m - 1, h->cgs_grid, h->cgs_cache, s));
+                                         h->d_H, J < m - 1, h->cgs_grid, h->cgs_cache, 0, brk_tol, s));
+            tick(h, GBPROP_PHASE_GRAM_SCHMIDT);
+            continue;
+        }
+        if (fused_dorth) {
+            GB_LAUNCH(launch_arnoldi_cgs(kp, V, nullptr, N, J, m, h->d_r, h->d_cgs_part, h->d_gridbar, h->d_ctrl, h->d_H,
+                                         1, h->cgs_dgrid, h->cgs_cache, 1, brk_tol, s));
             tick(h, GBPROP_PHASE_GRAM_SCHMIDT);
             continue;
         }
@@ -1082,12 +1090,12 @@ gbprop_status gbprop_finalize(gbprop_handle h) {
     // cooperative Gram-Schmidt (single handles; GBPROP_CGS=separate keeps the three-kernel form)
     {
         const char* env = std::getenv("GBPROP_CGS");
-        const bool allow = !(env && std::strcmp(env, "separate") == 0) && !h->double_orth;
+        const bool allow = !(env && std::strcmp(env, "separate") == 0);
         const int kpv = h->kprec(), with_v0 = h->d_v0 != nullptr;
-        int grid = allow ? arnoldi_cgs_grid(kpv, h->N, h->m, with_v0, 1) : 0;
+        int grid = allow ? arnoldi_cgs_grid(kpv, h->N, h->m, with_v0, 1, h->double_orth) : 0;
         int cache = 1;
         if (allow && grid == 0) {
-            grid = arnoldi_cgs_grid(kpv, h->N, h->m, with_v0, 0);
+            grid = arnoldi_cgs_grid(kpv, h->N, h->m, with_v0, 0, h->double_orth);
             cache = 0;
         }
         cudaGetLastError();
@@ -1096,7 +1104,7 @@ gbprop_status gbprop_finalize(gbprop_handle h) {
             h->cgs_part_grid = grid;
             if ((st = h->dalloc(&h->d_gridbar, 64))) return st;
             GB_CUDA(cudaMemsetAsync(h->d_gridbar, 0, 64, h->stream));
-            h->cgs_grid = grid;
+            (h->double_orth ? h->cgs_dgrid : h->cgs_grid) = grid;
             h->cgs_cache = cache;
         }
     }
@@ -1988,6 +1996,7 @@ gbprop_status gbprop_batch_create(gbprop_batch* out, const gbprop_handle* proble
                 h->cgs_part_grid = grid;
             }
             h->cgs_grid = grid;
+            h->cgs_dgrid = 0;
             h->cgs_cache = cache;
         }
         drop_graph(h);

@@ -20,6 +20,7 @@
 namespace gbprop {
 
 constexpr int kFuseThreads = 512;
+constexpr int kCgsMaxGrid = 256;               // partial sums per value (see to_fixed)
 constexpr long kBarrierSpinLimit = 1L << 24;   // polls (each an L2 round trip) before a barrier gives up
 
 // Grid barrier for a co-resident grid on a counter that only grows within an Arnoldi step
@@ -89,15 +90,53 @@ __device__ __forceinline__ void cgs_finish(Ctrl* ctrl, double* H, const double* 
     }
 }
 
-template <bool CACHE>
+// h[0..nvals) = sums over the CTAs' partials (two components per vector and CTA), every CTA the
+// same values: tpv threads per value, a power of two <= 32, so that a value's threads are
+// consecutive lanes of one warp; up to kRound partials per lane and round in fixed point.
+__device__ __forceinline__ void cgs_sum_partials(const double* part, int G, int nvals, double* h) {
+    constexpr int kRound = 10;
+    const int tid = threadIdx.x;
+    int tpv = 32;
+    while (tpv > 1 && tpv * nvals > kFuseThreads) tpv >>= 1;
+    const int v = tid / tpv, q = tid % tpv;
+    const double* p = part + (size_t)(v >> 1) * G * 2 + (v & 1);       // value v: component v & 1 of vector v >> 1
+    double total = 0.0;
+    for (int g0 = 0; g0 < G; g0 += kRound * tpv) {
+        double t[kRound];
+        int e = 0;
+#pragma unroll
+        for (int u = 0; u < kRound; ++u) {
+            const int g = g0 + q + u * tpv;
+            t[u] = v < nvals && g < G ? __ldcg(p + (size_t)g * 2) : 0.0;
+            e = max(e, exp_field(t[u]));
+        }
+        for (int o = 1; o < tpv; o <<= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+        long long f = 0;
+#pragma unroll
+        for (int u = 0; u < kRound; ++u) f += to_fixed<2>(t[u], e);
+        for (int o = 1; o < tpv; o <<= 1) f += shfl_xor_ll(f, o);
+        total = g0 ? total + from_fixed<2>(f, e) : from_fixed<2>(f, e);
+    }
+    if (v < nvals && q == 0) h[v] = total;
+}
+
+// DORTH: re-orthogonalisation inside the kernel (pamp.h:353-400): a pass is dot, barrier, update,
+// barrier, and every CTA takes the same decision from the same sums.  The column, the counters and the
+// next beta are then complete here (brk_tol: the happy-breakdown threshold), so the next solve
+// reads ctrl->inv_beta.  bar[1] holds the step's barriers used so far.  Against nine launches per Arnoldi step
+// (dot, update, three conditional passes of both, finalize), most of which find nothing to do:
+// a 16 x 300 step of m = 20 took 57 us of Gram-Schmidt per vector with those.
+template <bool CACHE, bool DORTH>
 __global__ void __launch_bounds__(kFuseThreads) k_arnoldi_cgs(const double2* __restrict__ V, long n, int J, int m,
                                                               double2* __restrict__ w, double* __restrict__ part,
                                                               unsigned* bar, Ctrl* ctrl, double* H, int update,
-                                                              int chunk) {
+                                                              int chunk, double brk_tol) {
     using C = double2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double hs[2 * (kMaxBasis + 1)];
+    __shared__ double ht[DORTH ? 2 * kMaxBasis : 1];   // the column, summed over the passes
     __shared__ double red[kFuseThreads / 32];
+    __shared__ int s_again;
     __shared__ __align__(8) unsigned long long s_bar;
     const int nv = J + 1, G = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long i0 = (long)b * chunk;
@@ -132,6 +171,7 @@ __global__ void __launch_bounds__(kFuseThreads) k_arnoldi_cgs(const double2* __r
         return;
     }
     const bool rnd = ctrl->round_matvec & 2;        // precision probe (FP64 handles)
+    unsigned tb = DORTH ? *(volatile const unsigned*)(bar + 1) : (unsigned)J;   // the step's next barrier
     if (tma) {
         if (tid == 0) {
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
@@ -147,119 +187,173 @@ __global__ void __launch_bounds__(kFuseThreads) k_arnoldi_cgs(const double2* __r
         for (int i = tid; i < cl; i += kFuseThreads) ws[i] = w[i0 + i];
         __syncthreads();
     }
-
-    // ---- phase A: partial inner products, one warp per basis vector.  The FP64 pipe retires
-    // one warp instruction per 16 SM cycles and its dependent latency is about as long, so two
-    // accumulator pairs per warp keep it busy; every extra add is pipe time. ----------------
-    for (int k = warp; k < nv; k += kFuseThreads / 32) {
-        double ar = 0.0, ai = 0.0, br = 0.0, bi = 0.0;
-        const C* vk = V + (size_t)k * n + i0;
-        int i = lane;
-        const C* ck = cache + (size_t)k * chunk;     // (staged rows when CACHE)
-        for (; i + 96 < cl; i += 128) {
-            C v[4];
+    double orig2 = 0.0, resid2 = 0.0;                  // warp 0: squared norms before and after a pass
+    double pre2 = 0.0;                                 // before the first
+    int passes = 0, again = 0;
+    for (;;) {
+        // ---- phase A: partial inner products, one warp per basis vector.  The FP64 pipe retires
+        // one warp instruction per 16 SM cycles and its dependent latency is about as long, so two
+        // accumulator pairs per warp keep it busy; the lanes' sums are added in fixed point. --------
+        for (int k = warp; k < nv; k += kFuseThreads / 32) {
+            double ar = 0.0, ai = 0.0, br = 0.0, bi = 0.0;
+            const C* vk = V + (size_t)k * n + i0;
+            int i = lane;
+            const C* ck = cache + (size_t)k * chunk;     // (staged rows when CACHE)
+            for (; i + 96 < cl; i += 128) {
+                C v[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = CACHE ? ck[i + 32 * u] : vk[i + 32 * u];
+                for (int u = 0; u < 4; ++u) v[u] = CACHE ? ck[i + 32 * u] : vk[i + 32 * u];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const C x = ws[i + 32 * u];
-                if (u & 1) acc_dot64(br, bi, v[u].x, v[u].y, x.x, x.y);
-                else acc_dot64(ar, ai, v[u].x, v[u].y, x.x, x.y);
+                for (int u = 0; u < 4; ++u) {
+                    const C x = ws[i + 32 * u];
+                    if (u & 1) acc_dot64(br, bi, v[u].x, v[u].y, x.x, x.y);
+                    else acc_dot64(ar, ai, v[u].x, v[u].y, x.x, x.y);
+                }
+            }
+            for (; i + 32 < cl; i += 64) {
+                const C v = CACHE ? ck[i] : vk[i], u = CACHE ? ck[i + 32] : vk[i + 32];
+                const C x = ws[i], y = ws[i + 32];
+                acc_dot64(ar, ai, v.x, v.y, x.x, x.y);
+                acc_dot64(br, bi, u.x, u.y, y.x, y.y);
+            }
+            if (i < cl) {
+                const C v = CACHE ? ck[i] : vk[i];
+                const C x = ws[i];
+                acc_dot64(ar, ai, v.x, v.y, x.x, x.y);
+            }
+            if (cl > 32) {
+                ar += br;
+                ai += bi;
+            }
+            ar = warp_fixed_sum(ar);
+            ai = warp_fixed_sum(ai);
+            if (lane == 0) {
+                part[((size_t)k * G + b) * 2] = ar;
+                part[((size_t)k * G + b) * 2 + 1] = ai;
             }
         }
-        for (; i + 32 < cl; i += 64) {
-            const C v = CACHE ? ck[i] : vk[i], u = CACHE ? ck[i + 32] : vk[i + 32];
-            const C x = ws[i], y = ws[i + 32];
-            acc_dot64(ar, ai, v.x, v.y, x.x, x.y);
-            acc_dot64(br, bi, u.x, u.y, y.x, y.y);
-        }
-        if (i < cl) {
-            const C v = CACHE ? ck[i] : vk[i];
-            const C x = ws[i];
-            acc_dot64(ar, ai, v.x, v.y, x.x, x.y);
-        }
-        ar += br;
-        ai += bi;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            ar += __shfl_xor_sync(0xffffffffu, ar, o);
-            ai += __shfl_xor_sync(0xffffffffu, ai, o);
-        }
-        if (lane == 0) {
-            part[((size_t)k * G + b) * 2] = ar;
-            part[((size_t)k * G + b) * 2 + 1] = ai;
-        }
-    }
-    if (!grid_barrier(bar, G, J, ctrl)) return;   // the launch's only barrier: number J of the step
-
-    // ---- phase B: h = sum of the partials (fixed order; tpv threads per value, a power of
-    // two <= 32 so that each value's threads are consecutive lanes of one warp) --------------
-    {
-        const int vals = 2 * nv;
-        int tpv = 32;
-        while (tpv > 1 && tpv * vals > kFuseThreads) tpv >>= 1;
-        const int v = tid / tpv, q = tid % tpv;
-        double s0 = 0.0, s1 = 0.0;
-        if (v < vals) {
-            const int k = v >> 1, c = v & 1;
-            const double* p = part + (size_t)k * G * 2 + c;
-            int g = q;
-            for (; g + tpv < G; g += 2 * tpv) {
-                s0 += __ldcg(p + (size_t)g * 2);
-                s1 += __ldcg(p + (size_t)(g + tpv) * 2);
-            }
-            if (g < G) s0 += __ldcg(p + (size_t)g * 2);
-        }
-        double s = s0 + s1;
-        for (int o = 1; o < tpv; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (v < vals && q == 0) hs[v] = s;
-    }
-    __syncthreads();
-
-    double nrm = 0.0;
-    if (update) {
-        // w -= V h on this chunk; ||w||^2 partial
-        for (int i = tid; i < cl; i += kFuseThreads) {
-            C r = ws[i];
-            double sr0 = 0.0, si0 = 0.0, sr1 = 0.0, si1 = 0.0;
-            int k = 0;
-            for (; k + 1 < nv; k += 2) {
-                const C a = CACHE ? cache[(size_t)k * chunk + i] : V[(size_t)k * n + i0 + i];
-                const C c = CACHE ? cache[(size_t)(k + 1) * chunk + i] : V[(size_t)(k + 1) * n + i0 + i];
-                sr0 = fma(a.x, hs[2 * k], sr0);
-                sr0 = fma(-a.y, hs[2 * k + 1], sr0);
-                si0 = fma(a.x, hs[2 * k + 1], si0);
-                si0 = fma(a.y, hs[2 * k], si0);
-                sr1 = fma(c.x, hs[2 * k + 2], sr1);
-                sr1 = fma(-c.y, hs[2 * k + 3], sr1);
-                si1 = fma(c.x, hs[2 * k + 3], si1);
-                si1 = fma(c.y, hs[2 * k + 2], si1);
-            }
-            if (k < nv) {
-                const C a = CACHE ? cache[(size_t)k * chunk + i] : V[(size_t)k * n + i0 + i];
-                sr0 = fma(a.x, hs[2 * k], sr0);
-                sr0 = fma(-a.y, hs[2 * k + 1], sr0);
-                si0 = fma(a.x, hs[2 * k + 1], si0);
-                si0 = fma(a.y, hs[2 * k], si0);
-            }
-            r.x -= (sr0 + sr1);
-            r.y -= (si0 + si1);
-            if (rnd) r = round_c64(r);
-            w[i0 + i] = r;
-            nrm = fma(r.x, r.x, nrm);
-            nrm = fma(r.y, r.y, nrm);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
-        if (lane == 0) red[warp] = nrm;
-        __syncthreads();
-        if (tid == 0) {
+        if (DORTH && passes == 0) {
+            // ||w||^2 before the first pass, as one more vector's partial
             double t = 0.0;
-            for (int q = 0; q < kFuseThreads / 32; ++q) t += red[q];
-            part[(size_t)nv * G * 2 + b] = t;     // beta is formed from these by the next solve
+            for (int i = tid; i < cl; i += kFuseThreads) {
+                const C x = ws[i];
+                t = fma(x.x, x.x, t);
+                t = fma(x.y, x.y, t);
+            }
+            t = warp_fixed_sum(t);
+            if (lane == 0) red[warp] = t;
+            __syncthreads();
+            if (warp == 0) {
+                t = warp_fixed_sum(lane < kFuseThreads / 32 ? red[lane] : 0.0);
+                if (lane == 0) {
+                    part[((size_t)nv * G + b) * 2] = t;
+                    part[((size_t)nv * G + b) * 2 + 1] = 0.0;
+                }
+            }
+        }
+        if (!grid_barrier(bar, G, tb++, ctrl)) return;
+
+        // ---- phase B: h = sum of the partials -----------------------------------------------
+        cgs_sum_partials(part, G, 2 * nv + (DORTH && passes == 0 ? 1 : 0), hs);
+        __syncthreads();
+        if (DORTH) {
+            if (passes == 0) pre2 = orig2 = hs[2 * nv];
+            for (int k = tid; k < 2 * nv; k += kFuseThreads) ht[k] = passes ? ht[k] + hs[k] : hs[k];
+        }
+
+        double nrm = 0.0;
+        if (update) {
+            // w -= V h on this chunk; ||w||^2 partial
+            for (int i = tid; i < cl; i += kFuseThreads) {
+                C r = ws[i];
+                double sr0 = 0.0, si0 = 0.0, sr1 = 0.0, si1 = 0.0;
+                int k = 0;
+                for (; k + 1 < nv; k += 2) {
+                    const C a = CACHE ? cache[(size_t)k * chunk + i] : V[(size_t)k * n + i0 + i];
+                    const C c = CACHE ? cache[(size_t)(k + 1) * chunk + i] : V[(size_t)(k + 1) * n + i0 + i];
+                    sr0 = fma(a.x, hs[2 * k], sr0);
+                    sr0 = fma(-a.y, hs[2 * k + 1], sr0);
+                    si0 = fma(a.x, hs[2 * k + 1], si0);
+                    si0 = fma(a.y, hs[2 * k], si0);
+                    sr1 = fma(c.x, hs[2 * k + 2], sr1);
+                    sr1 = fma(-c.y, hs[2 * k + 3], sr1);
+                    si1 = fma(c.x, hs[2 * k + 3], si1);
+                    si1 = fma(c.y, hs[2 * k + 2], si1);
+                }
+                if (k < nv) {
+                    const C a = CACHE ? cache[(size_t)k * chunk + i] : V[(size_t)k * n + i0 + i];
+                    sr0 = fma(a.x, hs[2 * k], sr0);
+                    sr0 = fma(-a.y, hs[2 * k + 1], sr0);
+                    si0 = fma(a.x, hs[2 * k + 1], si0);
+                    si0 = fma(a.y, hs[2 * k], si0);
+                }
+                r.x -= (sr0 + sr1);
+                r.y -= (si0 + si1);
+                if (rnd) r = make_double2(f2d_fast(d2f_fast(r.x)), f2d_fast(d2f_fast(r.y)));
+                if (DORTH) ws[i] = r;
+                else w[i0 + i] = r;
+                nrm = fma(r.x, r.x, nrm);
+                nrm = fma(r.y, r.y, nrm);
+            }
+            nrm = warp_fixed_sum(nrm);
+            if (lane == 0) red[warp] = nrm;
+            __syncthreads();
+            if (warp == 0) {
+                const double t = warp_fixed_sum(lane < kFuseThreads / 32 ? red[lane] : 0.0);
+                // (without DORTH: for the next solve's beta)
+                if (lane == 0) part[(size_t)(DORTH ? nv + 1 : nv) * G * 2 + b] = t;
+            }
+        }
+        if (!DORTH) break;
+        if (!grid_barrier(bar, G, tb++, ctrl)) return;
+        if (warp == 0) {
+            const double t = warp_fixed_sum_of(part + (size_t)(nv + 1) * G * 2, G, 1);
+            if (passes > 0) orig2 = resid2;
+            resid2 = t;
+            if (lane == 0) s_again = t < 0.717 * 0.717 * orig2;      // pamp.h:369
+        }
+        __syncthreads();
+        again = s_again;
+        // the reference loop runs at most MaxOrthogonalizationCount = 3 passes (pamp.h:75,375)
+        if (!again || passes == 3) break;
+        ++passes;
+    }
+    if constexpr (!DORTH) {
+        cgs_finish(ctrl, H, hs, m, J, b);
+    } else {
+        for (int i = tid; i < cl; i += kFuseThreads) w[i0 + i] = ws[i];
+        if (b != 0) return;
+        for (int k = tid; k < nv; k += kFuseThreads) {
+            H[2 * ((size_t)k * m + J)] = ht[2 * k];
+            H[2 * ((size_t)k * m + J) + 1] = ht[2 * k + 1];
+            ctrl->h[2 * k] = ht[2 * k];
+            ctrl->h[2 * k + 1] = ht[2 * k + 1];
+        }
+        if (tid != 0) return;
+        const double resid = sqrt(resid2);
+        bar[1] = tb;
+        ctrl->nbasis = nv;
+        ctrl->operator_count++;
+        if (J == 0) ctrl->inner_product_count++;
+        // after the third pass the reference counts once more and stops (pamp.h:372-381)
+        ctrl->orthogonalization_count += passes + (again && passes == 3 ? 1 : 0);
+        ctrl->ro_count = passes;
+        ctrl->ro_go = again;
+        ctrl->pre_norm = sqrt(pre2);
+        ctrl->orig_norm = sqrt(orig2);
+        ctrl->resid_norm = resid;
+        if (!isfinite(resid)) ctrl->nonfinite = 1;
+        if (J + 1 >= m) return;
+        if (fabs(resid) < brk_tol) {
+            ctrl->broken = 1;
+            ctrl->breakdown_count++;
+        } else {
+            H[2 * ((size_t)(J + 1) * m + J)] = resid;
+            H[2 * ((size_t)(J + 1) * m + J) + 1] = 0.0;
+            ctrl->beta = resid;
+            set_inv_beta(ctrl, resid);
         }
     }
-    cgs_finish(ctrl, H, hs, m, J, b);
 }
 
 // ---------------------------------------------------------------------------
@@ -522,6 +616,11 @@ size_t arnoldi_cgs_smem(int prec, long n, int nv, int grid, int with_v0, int cac
     return b;
 }
 
+static decltype(&k_arnoldi_cgs<true, false>) cgs_kernel64(int cache, int dorth) {
+    return dorth ? (cache ? k_arnoldi_cgs<true, true> : k_arnoldi_cgs<false, true>)
+                 : (cache ? k_arnoldi_cgs<true, false> : k_arnoldi_cgs<false, false>);
+}
+
 template <typename Kern, typename... Args>
 static cudaError_t cgs_coop_launch(Kern kern, int grid, size_t smem, cudaStream_t s, Args... args) {
     cudaError_t e = allow_max_smem(kern);
@@ -543,35 +642,38 @@ static cudaError_t cgs_coop_launch(Kern kern, int grid, size_t smem, cudaStream_
 
 cudaError_t launch_arnoldi_cgs(int prec, const void* V, const void* v0, long n, int J, int m, void* w,
                                double* part, unsigned* bar, Ctrl* ctrl, double* H, int update, int grid, int cache,
-                               cudaStream_t s) {
+                               int dorth, double brk_tol, cudaStream_t s) {
     count_launch();
     const int chunk = (int)(((n + grid - 1) / grid + 7) / 8 * 8);
     const size_t smem = arnoldi_cgs_smem(prec, n, J + 1, grid, v0 != nullptr, cache);
     if (prec == 0) {
-        auto kern = cache ? k_arnoldi_cgs<true> : k_arnoldi_cgs<false>;
+        auto kern = cgs_kernel64(cache, dorth);
         return cgs_coop_launch(kern, grid, smem, s, (const double2*)V, n, J, m, (double2*)w, part, bar, ctrl, H, update,
-                               chunk);
+                               chunk, brk_tol);
     }
+    if (dorth) return cudaErrorInvalidValue;
     auto kern = cache ? k_arnoldi_cgs32<true> : k_arnoldi_cgs32<false>;
     return cgs_coop_launch(kern, grid, smem, s, (const float2*)V, (const float4*)v0, n, J, m, (float2*)w,
                            (float4*)part, bar, ctrl, H, update, chunk);
 }
 
-// Largest grid of co-resident CTAs for this configuration (0 when the cooperative form
-// cannot run: no cooperative launch support or shared memory too large).
-int arnoldi_cgs_grid(int prec, long n, int m, int with_v0, int cache) {
+// Grid of co-resident CTAs for this configuration: one CTA per SM, or one per 32 elements where
+// those are fewer -- a warp of a smaller chunk takes as long, and every CTA sums all CTAs' partials
+// (0 when the cooperative form cannot run: no cooperative launch support or shared memory too large).
+int arnoldi_cgs_grid(int prec, long n, int m, int with_v0, int cache, int dorth) {
     int dev = 0, sms = 0, coop = 0, optin = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (!coop || sms <= 0) return 0;
-    const size_t smem = arnoldi_cgs_smem(prec, n, m, sms, with_v0, cache);
-    if (smem + 4096 > (size_t)optin) return 0;
+    if (!coop || sms <= 0 || (dorth && prec != 0)) return 0;
+    const int grid = (int)std::min<long>(std::min(sms, kCgsMaxGrid), std::max<long>(1, (n + 31) / 32));
+    const size_t smem = arnoldi_cgs_smem(prec, n, m, grid, with_v0, cache);
+    if (smem + 8192 > (size_t)optin) return 0;
     int per_sm = 0;
     cudaError_t e;
     if (prec == 0) {
-        auto kern = cache ? k_arnoldi_cgs<true> : k_arnoldi_cgs<false>;
+        auto kern = cgs_kernel64(cache, dorth);
         allow_max_smem(kern);
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFuseThreads, smem);
     } else {
@@ -581,7 +683,7 @@ int arnoldi_cgs_grid(int prec, long n, int m, int with_v0, int cache) {
     }
     cudaGetLastError();
     if (e != cudaSuccess || per_sm < 1) return 0;
-    return sms;
+    return grid;
 }
 
 // Grid of the cooperative form for a problem inside a batch, where other problems fill the
@@ -594,6 +696,7 @@ int arnoldi_cgs_grid_batch(int prec, long n, int m, int with_v0, int* cache) {
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (!coop || sms <= 0) return 0;
+    sms = std::min(sms, kCgsMaxGrid);
     for (int c = 1; c >= 0; --c) {
         int grid = c ? 1 : (int)std::min<long>(sms, std::max<long>(1, (n + 2047) / 2048));
         if (c)
@@ -604,7 +707,7 @@ int arnoldi_cgs_grid_batch(int prec, long n, int m, int with_v0, int* cache) {
         int per_sm = 0;
         cudaError_t e;
         if (prec == 0) {
-            auto kern = c ? k_arnoldi_cgs<true> : k_arnoldi_cgs<false>;
+            auto kern = cgs_kernel64(c, 0);
             allow_max_smem(kern);
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFuseThreads, smem);
         } else {

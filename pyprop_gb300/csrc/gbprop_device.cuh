@@ -312,17 +312,83 @@ __device__ __forceinline__ float2 inv_sqrt_pair(float th, float tl) {
     return make_float2(s, e);
 }
 
-// beta = ||w|| of the next basis vector from the FP64 cooperative Gram-Schmidt kernel's per-CTA
-// ||w||^2 partials (one double per CTA), summed by one warp in a fixed order (the same beta in every
-// CTA that calls it).  Whole warp; returns beta in every lane.
-__device__ __forceinline__ double gs_beta(const void* part, int G) {
-    const int lane = threadIdx.x & 31;
-    const double* p = reinterpret_cast<const double*>(part);
-    double t = 0.0;
-    for (int g = lane; g < G; g += 32) t += __ldcg(p + g);
+// ---------------------------------------------------------------------------
+// Sums of FP64 values as 64-bit fixed-point numbers.  An FP64 add occupies its SM sub-partition for
+// 64 cycles per warp whatever its lanes do, so a butterfly of them costs what the products of a
+// Gram-Schmidt step cost; integer adds issue 30 times as fast.  Every value is taken at the exponent
+// of the largest, with S bits below its last (so up to 2^(10 - S) values fit; 2^-(53 + S) of the
+// largest is each value's only rounding); the result does not depend on the order.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ int exp_field(double d) { return (__double2hiint(d) >> 20) & 0x7ff; }
+
+// d * 2^(1075 + S - emax) rounded to an integer, |result| < 2^(53 + S); emax >= exp_field(d); subnormals
+// are zero
+template <int S>
+__device__ __forceinline__ long long to_fixed(double d, int emax) {
+    const int hi = __double2hiint(d), ef = (hi >> 20) & 0x7ff, s = emax - ef;
+    const unsigned long long m = ((unsigned long long)(((unsigned)hi & 0xfffffu) | 0x100000u) << (32 + S)) |
+                                 ((unsigned long long)(unsigned)__double2loint(d) << S);
+    const long long v = ef == 0 || s > 53 + S ? 0 : (long long)((m + ((1ull << s) >> 1)) >> s);
+    return hi < 0 ? -v : v;
+}
+
+// the double nearest to f * 2^(emax - 1075 - S); NaN where emax was that of an infinity or a NaN
+template <int S>
+__device__ __forceinline__ double from_fixed(long long f, int emax) {
+    const unsigned long long a = f < 0 ? (unsigned long long)-f : (unsigned long long)f;
+    const int lz = __clzll((long long)a), e = emax + 11 - S - lz;
+    if (emax == 2047) return __hiloint2double(0x7ff80000, 0);
+    if (a == 0 || e <= 0) return 0.0;
+    if (e >= 2047) return __hiloint2double(f < 0 ? 0xfff00000 : 0x7ff00000, 0);
+    const unsigned long long n = a << lz;              // leading one at bit 63
+    const unsigned long long m = (n >> 11) + ((n >> 10) & 1);
+    const unsigned long long bits = m + ((unsigned long long)(e - 1) << 52);   // (adds the implicit bit's carry)
+    return __longlong_as_double((long long)(bits | (f < 0 ? 0x8000000000000000ull : 0ull)));
+}
+
+__device__ __forceinline__ long long shfl_xor_ll(long long v, int o) {
+    const int lo = __shfl_xor_sync(0xffffffffu, (int)v, o), hi = __shfl_xor_sync(0xffffffffu, (int)(v >> 32), o);
+    return ((long long)hi << 32) | (unsigned)lo;
+}
+
+// the warp's sum in every lane
+__device__ __forceinline__ double warp_fixed_sum(double v) {
+    const int e = (int)__reduce_max_sync(0xffffffffu, (unsigned)exp_field(v));
+    long long f = to_fixed<3>(v, e);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    return sqrt(t);
+    for (int o = 16; o > 0; o >>= 1) f += shfl_xor_ll(f, o);
+    return from_fixed<3>(f, e);
+}
+
+// the warp's sum of p[0], p[stride], ... (count values), in every lane: up to 8 per lane at once
+__device__ __forceinline__ double warp_fixed_sum_of(const double* p, int count, int stride) {
+    const int lane = threadIdx.x & 31;
+    double total = 0.0;
+    for (int g0 = 0; g0 < count; g0 += 256) {
+        double t[8];
+        int e = 0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int g = g0 + lane + 32 * u;
+            t[u] = g < count ? __ldcg(p + (size_t)g * stride) : 0.0;
+            e = max(e, exp_field(t[u]));
+        }
+        e = (int)__reduce_max_sync(0xffffffffu, (unsigned)e);
+        long long f = 0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) f += to_fixed<2>(t[u], e);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) f += shfl_xor_ll(f, o);
+        total = g0 ? total + from_fixed<2>(f, e) : from_fixed<2>(f, e);
+    }
+    return total;
+}
+
+// beta = ||w|| of the next basis vector from the FP64 cooperative Gram-Schmidt kernel's per-CTA
+// ||w||^2 partials (one double per CTA), summed by one warp (the same beta in every CTA that calls
+// it).  Whole warp; returns beta in every lane.
+__device__ __forceinline__ double gs_beta(const void* part, int G) {
+    return sqrt(warp_fixed_sum_of(reinterpret_cast<const double*>(part), G, 1));
 }
 
 // Records beta of the next basis vector (pamp.h:330-345; happy breakdown below sqrt(eps),

@@ -257,13 +257,15 @@ cudaError_t launch_arnoldi_finalize(Ctrl* ctrl, double* H, int m, int J, int dou
 // arnoldi_cgs_part_doubles(grid) doubles; bar: two words, zero before the first launch.
 // update = 0 forms only the Hessenberg column (last vector).  cache: keep V's chunk in
 // shared memory between the two passes.
+// dorth (FP64): re-orthogonalisation passes inside, and the column, the next beta and the breakdown
+// test (brk_tol) complete on return, as launch_arnoldi_finalize leaves them.
 // The complex64 form takes the first vector as FP32 pairs (v0s, see launch_solve_inv) and
 // forms every sum with error-free FP32 transformations.
 cudaError_t launch_arnoldi_cgs(int prec, const void* V, const void* v0, long n, int J, int m, void* w,
                                double* part, unsigned* bar, Ctrl* ctrl, double* H, int update, int grid, int cache,
-                               cudaStream_t s);
+                               int dorth, double brk_tol, cudaStream_t s);
 // Grid size for the cooperative Gram-Schmidt (0 if it cannot run co-resident).
-int arnoldi_cgs_grid(int prec, long n, int m, int with_v0, int cache);
+int arnoldi_cgs_grid(int prec, long n, int m, int with_v0, int cache, int dorth);
 int arnoldi_cgs_grid_batch(int prec, long n, int m, int with_v0, int* cache);
 inline size_t arnoldi_cgs_part_doubles(int grid) { return (size_t)(2 * (kMaxBasis + 1) + 1) * grid; }
 cudaError_t launch_step_begin(Ctrl* ctrl, double* H, int m, cudaStream_t s);
