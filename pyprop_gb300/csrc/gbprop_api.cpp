@@ -516,6 +516,17 @@ gbprop_status upload_band_op(gbprop_ctx* h, const HostBandOp& ho, BandOp<T>* out
     out->t_coef = coef;
     out->slots = slots;
     out->slots_lo = nullptr;
+    // per-row descriptors (build_band_op's factors are 1 or i)
+    int maxt = 0;
+    for (int l = 0; l < h->nl; ++l) maxt = std::max(maxt, ho.row_ptr[l + 1] - ho.row_ptr[l]);
+    std::vector<int4> desc(std::max<size_t>(1, (size_t)h->nl * maxt), make_int4(-1, 0, 0, 0));
+    for (int l = 0; l < h->nl; ++l)
+        for (int t = ho.row_ptr[l]; t < ho.row_ptr[l + 1]; ++t)
+            desc[(size_t)l * maxt + t - ho.row_ptr[l]] = make_int4(ho.src[t], ho.slot[t], ho.timedep[t], ho.coef[2 * t + 1] != 0.0);
+    int4* dd;
+    if ((st = h->upload(&dd, desc))) return st;
+    out->maxt = maxt;
+    out->desc = dd;
     if (sizeof(T) < sizeof(double)) {
         // complex64 path: the rounding remainder of every coefficient, so the operator
         // applied is the FP64 one (to ~2^-48) and only the FP32 sums round

@@ -132,6 +132,10 @@ template <typename T> struct BandOp {
     const double* t_coef;    // 2 * nterms (re, im)
     const T* slots;
     const T* slots_lo;       // FP32 only: slot - (float)slot, the coefficients' rounding remainder
+    // the same terms as nl x maxt descriptors: source row (-1: none), slot, time function (0: static), 1
+    // where the factor is i instead of 1
+    int maxt;
+    const int4* desc;
 };
 
 // Device control block of one handle.  Every field is written by kernels only, except

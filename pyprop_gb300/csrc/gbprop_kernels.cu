@@ -21,6 +21,7 @@
 #include <cstdlib>
 #include <cfloat>
 #include <cmath>
+#include <type_traits>
 
 namespace gbprop {
 
@@ -153,8 +154,8 @@ __device__ void block_partials<16>(double (&acc)[16], int nvalid, double* partia
 // (threads per block, radial elements per thread).
 // Variants 4 and 5 stage nothing: one thread per element reads its stencil through L1.
 // Variants 6, 7, 8 (even nr): two elements per thread with vector loads (k_band_apply_x2 / _x2d;
-// 128, 64, 32 threads).
-constexpr int kBandVariants = 9;
+// 128, 64, 32 threads).  Variants 9, 10: a lane per component, a warp per term (k_band_split).
+constexpr int kBandVariants = 11;
 __host__ __device__ constexpr int band_threads(int v) {
     return v == 0 ? 64 : v == 1 ? 128 : v == 2 ? 128 : v == 3 ? 256 : v == 4 ? 128 : 256;
 }
@@ -565,11 +566,137 @@ __global__ void __launch_bounds__(THREADS) k_band_apply_x2d(BandOp<double> op, c
     }
 }
 
-bool band_variant_vec_ok(int v, int nr) { return v < 6 || nr % 2 == 0; }
+// One lane per element and component, one warp per term (variants 9 and 10: 1 or 2 groups of 16
+// elements per warp).  A term's band is real, so the two components of an element are independent
+// sums of 2 KB + 1 products; the terms of a row go to different warps of the CTA and meet in shared
+// memory.  An FP64 instruction holds its SM sub-partition for 64 cycles whatever its lanes do, so what
+// counts is how evenly the warp instructions fall on the 608 sub-partitions: against one thread per
+// element or pair of elements that walks through its row's terms this has six times as many warps of a
+// sixth of the length, and their loads are in flight together instead of term after term.  A warp's
+// descriptor is one 16-byte load; nothing depends on the row table.
+constexpr int kTermWarps = 4;
+template <typename T, int KB, int G>
+__global__ void __launch_bounds__(32 * kTermWarps) k_band_split(BandOp<T> op, const T* __restrict__ x,
+                                                                T* __restrict__ y, const SchedEntry* __restrict__ sched,
+                                                                const Ctrl* __restrict__ ctrl, Scalings scal_val,
+                                                                int check_broken) {
+    constexpr int W = 2 * KB + 1;
+    constexpr bool F64 = sizeof(T) == sizeof(double);
+    using S = typename std::conditional<F64, double, float2>::type;     // a term's share: FP64, or an FP32 pair
+    __shared__ S part[kTermWarps][G][32];
+    const int l = blockIdx.y, nr = op.nr, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tw = blockDim.x >> 5;
+    const int i0 = blockIdx.x * 16 * G + (lane >> 1), c = lane & 1;
+    const int4* desc = op.desc + (size_t)l * op.maxt;
+    int4 ds = __ldg(desc + warp);                     // (blockDim.x / 32 <= maxt)
+    pdl_wait();
+    const int skip = check_broken ? ctrl->broken : 0;
+    const int probe = F64 && ctrl ? ctrl->round_matvec : 0;
+    const SchedEntry* now = sched ? sched + ctrl->step : nullptr;
+    S acc[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        if constexpr (F64) acc[g] = 0.0;
+        else acc[g] = make_float2(0.f, 0.f);
+    }
+    for (int t = warp; ds.x >= 0;) {
+        const T* xs = x + 2 * (size_t)ds.x * nr + c;
+        const size_t so = (size_t)ds.y * W * nr;
+        const double f = ds.z ? (now ? now->scaling.s[ds.z - 1] : scal_val.s[ds.z - 1]) : 1.0;
+        T a[G][W], v[G][W], al[G][F64 ? 1 : W];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const int i = i0 + 16 * g;
+#pragma unroll
+            for (int d = 0; d < W; ++d) {
+                const int j = i + d - KB;
+                a[g][d] = i < nr ? __ldg(op.slots + so + (size_t)d * nr + i) : T(0);
+                if constexpr (!F64) al[g][d] = i < nr ? __ldg(op.slots_lo + so + (size_t)d * nr + i) : T(0);
+                v[g][d] = j >= 0 && j < nr ? __ldg(xs + 2 * j) : T(0);
+            }
+        }
+        const bool imag = ds.w != 0;
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            if constexpr (F64) {
+                double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+                for (int d = 0; d < W; ++d) {
+                    if (d & 1) s1 = fma(a[g][d], v[g][d], s1);
+                    else s0 = fma(a[g][d], v[g][d], s0);
+                }
+                double s = s0 + s1;
+                if (imag) {
+                    // i f s: the real part's sum goes to the imaginary component, the other back negated
+                    s = __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(s), 1),
+                                         __shfl_xor_sync(0xffffffffu, __double2loint(s), 1));
+                    if (c == 0) s = __hiloint2double(__double2hiint(s) ^ 0x80000000, __double2loint(s));
+                }
+                if (ds.z) acc[g] = fma(f, s, acc[g]);
+                else acc[g] += s;
+            } else {
+                // error-free products, compensated sums (even and odd diagonals apart), as the other forms
+                float sh = 0.f, sl = 0.f, oh = 0.f, ol = 0.f;
+#pragma unroll
+                for (int d = 0; d < W; ++d) {
+                    if (d & 1) acc_prod(oh, ol, a[g][d], al[g][d], v[g][d]);
+                    else acc_prod(sh, sl, a[g][d], al[g][d], v[g][d]);
+                }
+                acc_pair(sh, sl, oh, ol);
+                if (imag) {
+                    sh = __shfl_xor_sync(0xffffffffu, sh, 1);
+                    sl = __shfl_xor_sync(0xffffffffu, sl, 1);
+                    if (c == 0) { sh = -sh; sl = -sl; }
+                }
+                if (ds.z) {
+                    const float fh = (float)f, fl = (float)(f - (double)fh);
+                    acc_scaled(acc[g].x, acc[g].y, fh, fl, sh, sl);
+                } else {
+                    acc_pair(acc[g].x, acc[g].y, sh, sl);
+                }
+            }
+        }
+        t += tw;
+        if (t >= op.maxt) break;
+        ds = __ldg(desc + t);
+    }
+    if (skip) return;                                 // uniform: written only between launches
+#pragma unroll
+    for (int g = 0; g < G; ++g) part[warp][g][lane] = acc[g];
+    __syncthreads();
+    for (int g = warp; g < G; g += tw) {
+        const int i = i0 + 16 * g;
+        if (i >= nr) continue;
+        T out;
+        if constexpr (F64) {
+            double s = part[0][g][lane];
+            for (int q = 1; q < tw; ++q) s += part[q][g][lane];
+            out = (probe & 1) ? f2d_fast(d2f_fast(s)) : s;
+        } else {
+            float2 s = part[0][g][lane];
+            for (int q = 1; q < tw; ++q) acc_pair(s.x, s.y, part[q][g][lane].x, part[q][g][lane].y);
+            out = s.x + s.y;
+        }
+        y[2 * ((size_t)l * nr + i) + c] = out;
+    }
+}
+
+bool band_variant_vec_ok(int v, int nr) { return v < 6 || v > 8 || nr % 2 == 0; }
 
 template <typename T, int KB, int V>
 static void band_apply_v(const BandOp<T>& op, const void* x, void* y, const SchedEntry* sched, const Ctrl* ctrl,
                          const Scalings& scaling, int check_broken, cudaStream_t s) {
+    if constexpr (V >= 9) {
+        constexpr int G = V == 9 ? 1 : 2;
+        if (sizeof(T) == sizeof(double) || op.slots_lo) {
+            const int tw = op.maxt < kTermWarps ? (op.maxt < 1 ? 1 : op.maxt) : kTermWarps;
+            dim3 grid((op.nr + 16 * G - 1) / (16 * G), op.nl);
+            launch_pdl(k_band_split<T, KB, G>, grid, dim3(32 * tw), 0, s, op, (const T*)x, (T*)y, sched, ctrl, scaling,
+                       check_broken);
+            return;
+        }
+        band_apply_v<T, KB, 4>(op, x, y, sched, ctrl, scaling, check_broken, s);
+        return;
+    }
     if constexpr (V >= 6) {
         // (selected by the host only for complex64 operators with split coefficients and even nr;
         // vectors not on a 16-byte boundary take the one-element form)
@@ -619,6 +746,8 @@ static void band_apply_kb(const BandOp<T>& op, const void* x, void* y, const Sch
         case 6: band_apply_v<T, KB, 6>(op, x, y, sched, ctrl, scaling, check_broken, s); break;
         case 7: band_apply_v<T, KB, 7>(op, x, y, sched, ctrl, scaling, check_broken, s); break;
         case 8: band_apply_v<T, KB, 8>(op, x, y, sched, ctrl, scaling, check_broken, s); break;
+        case 9: band_apply_v<T, KB, 9>(op, x, y, sched, ctrl, scaling, check_broken, s); break;
+        case 10: band_apply_v<T, KB, 10>(op, x, y, sched, ctrl, scaling, check_broken, s); break;
         default: band_apply_v<T, KB, 1>(op, x, y, sched, ctrl, scaling, check_broken, s); break;
     }
 }
