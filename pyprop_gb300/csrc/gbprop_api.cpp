@@ -527,6 +527,18 @@ gbprop_status upload_band_op(gbprop_ctx* h, const HostBandOp& ho, BandOp<T>* out
     if ((st = h->upload(&dd, desc))) return st;
     out->maxt = maxt;
     out->desc = dd;
+    out->fslots = nullptr;
+    out->fexp = nullptr;
+    if (sizeof(T) == sizeof(double) && !ho.slots.empty()) {
+        const int W = 2 * ho.kb + 1, nslots = (int)(ho.slots.size() / ((size_t)W * h->nr));
+        int2* fs;
+        int* fe;
+        if ((st = h->dalloc(&fs, ho.slots.size() * sizeof(int2)))) return st;
+        if ((st = h->dalloc(&fe, (size_t)nslots * h->nr * sizeof(int)))) return st;
+        GB_CUDA(launch_band_fixed_slots((const double*)slots, nslots, h->nr, W, fs, fe, h->stream));
+        out->fslots = fs;
+        out->fexp = fe;
+    }
     if (sizeof(T) < sizeof(double)) {
         // complex64 path: the rounding remainder of every coefficient, so the operator
         // applied is the FP64 one (to ~2^-48) and only the FP32 sums round
@@ -1405,6 +1417,7 @@ gbprop_status gbprop_tensor_multiply_bandnh(int storage, const void* V, int npai
 bool band_variant_available(const gbprop_ctx* h, int v) {
     if (v < 0 || v >= band_variant_count()) return false;
     if (v < 6) return true;
+    if (v >= 11) return h->kprec() == 0 && h->t64.op.fslots != nullptr;
     if (!band_variant_vec_ok(v, h->nr)) return false;
     return h->kprec() == 0 || h->t32.op.slots_lo != nullptr;
 }

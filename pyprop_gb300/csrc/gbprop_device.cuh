@@ -346,6 +346,26 @@ __device__ __forceinline__ double from_fixed(long long f, int emax) {
     return __longlong_as_double((long long)(bits | (f < 0 ? 0x8000000000000000ull : 0ull)));
 }
 
+// the double nearest to (hi 2^64 + lo) 2^e, hi and lo one two's complement number
+__device__ __forceinline__ double from_fixed128(long long hi, unsigned long long lo, int e) {
+    const bool neg = hi < 0;
+    unsigned long long h = (unsigned long long)hi;
+    if (neg) {
+        lo = 0ull - lo;
+        h = ~h + (lo == 0);
+    }
+    const int lz = h ? __clzll((long long)h) : 64 + __clzll((long long)lo);
+    if (lz == 128) return 0.0;
+    // leading one at bit 63
+    const unsigned long long n = lz == 0 ? h : lz < 64 ? (h << lz) | (lo >> (64 - lz)) : lo << (lz - 64);
+    const int f = 127 - lz + e + 1023;
+    if (f <= 0) return 0.0;
+    if (f >= 2047) return __hiloint2double(neg ? 0xfff00000 : 0x7ff00000, 0);
+    const unsigned long long m = (n >> 11) + ((n >> 10) & 1);
+    const unsigned long long bits = m + ((unsigned long long)(f - 1) << 52);
+    return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
+}
+
 __device__ __forceinline__ long long shfl_xor_ll(long long v, int o) {
     const int lo = __shfl_xor_sync(0xffffffffu, (int)v, o), hi = __shfl_xor_sync(0xffffffffu, (int)(v >> 32), o);
     return ((long long)hi << 32) | (unsigned)lo;

@@ -136,6 +136,9 @@ template <typename T> struct BandOp {
     // where the factor is i instead of 1
     int maxt;
     const int4* desc;
+    // FP64: the slots as 58-bit fixed-point numbers (see split29) at each row's largest exponent
+    const int2* fslots;
+    const int* fexp;         // nslots x nr
 };
 
 // Device control block of one handle.  Every field is written by kernels only, except
@@ -296,6 +299,9 @@ cudaError_t launch_zero(void* p, size_t bytes, cudaStream_t s);
 
 int grid_reduce_blocks();
 int band_variant_count();
+// fixed-point form of FP64 slots (nslots x (2 kb + 1) x nr) and the row exponents (nslots x nr)
+cudaError_t launch_band_fixed_slots(const double* slots, int nslots, int nr, int width, int2* digits, int* exps,
+                                    cudaStream_t s);
 bool band_variant_vec_ok(int v, int nr);    // the variant's radial-size condition (even nr for 6, 7, 8)
 // Bound states of banded generalized symmetric problems (gbprop_bound.cu; see gbprop_bound_states)
 cudaError_t launch_bound_states(const double* Hb, const double* Sb, int n, int kd, int nrows, double emax,

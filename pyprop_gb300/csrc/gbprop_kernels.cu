@@ -155,7 +155,7 @@ __device__ void block_partials<16>(double (&acc)[16], int nvalid, double* partia
 // Variants 4 and 5 stage nothing: one thread per element reads its stencil through L1.
 // Variants 6, 7, 8 (even nr): two elements per thread with vector loads (k_band_apply_x2 / _x2d;
 // 128, 64, 32 threads).  Variants 9, 10: a lane per component, a warp per term (k_band_split).
-constexpr int kBandVariants = 11;
+constexpr int kBandVariants = 13;
 __host__ __device__ constexpr int band_threads(int v) {
     return v == 0 ? 64 : v == 1 ? 128 : v == 2 ? 128 : v == 3 ? 256 : v == 4 ? 128 : 256;
 }
@@ -680,13 +680,154 @@ __global__ void __launch_bounds__(32 * kTermWarps) k_band_split(BandOp<T> op, co
     }
 }
 
+// The same split in 58-bit fixed point (variants 11 and 12: 1 or 2 groups of 16 elements per warp).
+// A product of FP64 numbers is one FP64 instruction, 64 cycles of its sub-partition, but three
+// integer multiply-adds of 2 each: with a = a1 2^29 + a0 and x = x1 2^29 + x0 in signed digits,
+//     a x = a1 x1 2^58 + (a1 x0 + a0 x1) 2^29 + a0 x0,
+// the last of which, 2^-60 of the largest product, is left out.  Coefficients are at the exponent of their
+// row's largest, x at that of the largest entry a warp reads (16 G + 2 KB elements), so a row errs by
+// 2^-58 of the largest coefficient times the largest entry and each product, where FP64 rounds every
+// partial sum to 2^-53.
+constexpr int kFixedBits = 58;
+__device__ __forceinline__ int2 split29(long long f) {
+    const int lo = ((int)(unsigned)f << 3) >> 3;
+    return make_int2((int)((f - lo) >> 29), lo);
+}
+
+__global__ void k_band_fixed_slots(const double* __restrict__ slots, int nr, int width, int2* __restrict__ digits,
+                                   int* __restrict__ exps) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nr) return;
+    const size_t so = (size_t)blockIdx.y * width * nr + i;
+    int e = 0;
+    for (int d = 0; d < width; ++d) e = max(e, exp_field(slots[so + (size_t)d * nr]));
+    for (int d = 0; d < width; ++d)
+        digits[so + (size_t)d * nr] = split29(to_fixed<kFixedBits - 53>(slots[so + (size_t)d * nr], e));
+    exps[(size_t)blockIdx.y * nr + i] = e;
+}
+
+cudaError_t launch_band_fixed_slots(const double* slots, int nslots, int nr, int width, int2* digits, int* exps,
+                                    cudaStream_t s) {
+    for (int k = 0; k < nslots; k += 65535) {
+        const int n = std::min(65535, nslots - k);
+        const size_t o = (size_t)k * width * nr;
+        k_band_fixed_slots<<<dim3((nr + 127) / 128, n), 128, 0, s>>>(slots + o, nr, width, digits + o, exps + (size_t)k * nr);
+    }
+    return cudaGetLastError();
+}
+
+template <int KB, int G>
+__global__ void __launch_bounds__(32 * kTermWarps) k_band_fixed(BandOp<double> op, const double* __restrict__ x,
+                                                                double* __restrict__ y,
+                                                                const SchedEntry* __restrict__ sched,
+                                                                const Ctrl* __restrict__ ctrl, Scalings scal_val,
+                                                                int check_broken) {
+    constexpr int W = 2 * KB + 1, NV = 2 * (16 * G + 2 * KB), NX = (NV + 31) / 32;
+    __shared__ int2 xf[kTermWarps][NV];
+    __shared__ double part[kTermWarps][G][32];
+    const int l = blockIdx.y, nr = op.nr, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tw = blockDim.x >> 5;
+    const int t0 = blockIdx.x * 16 * G, i0 = t0 + (lane >> 1), c = lane & 1;
+    const int4* desc = op.desc + (size_t)l * op.maxt;
+    int4 ds = __ldg(desc + warp);                     // (blockDim.x / 32 <= maxt)
+    int2 a[G][W];
+    int ea[G];
+    auto load = [&](int slot) {
+        const size_t so = (size_t)slot * W * nr;
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const int i = i0 + 16 * g;
+#pragma unroll
+            for (int d = 0; d < W; ++d)
+                a[g][d] = i < nr ? __ldg(op.fslots + so + (size_t)d * nr + i) : make_int2(0, 0);
+            ea[g] = i < nr ? __ldg(op.fexp + (size_t)slot * nr + i) : 0;
+        }
+    };
+    if (ds.x >= 0) load(ds.y);
+    pdl_wait();
+    const int skip = check_broken ? ctrl->broken : 0;
+    const int probe = ctrl ? ctrl->round_matvec : 0;
+    const SchedEntry* now = sched ? sched + ctrl->step : nullptr;
+    double acc[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) acc[g] = 0.0;
+    for (int t = warp; ds.x >= 0;) {
+        const double* xs = x + 2 * (size_t)ds.x * nr;
+        const double f = ds.z ? (now ? now->scaling.s[ds.z - 1] : scal_val.s[ds.z - 1]) : 1.0;
+        double v[NX];
+        int ex = 0;
+#pragma unroll
+        for (int u = 0; u < NX; ++u) {
+            const int q = lane + 32 * u, j = 2 * (t0 - KB) + q;
+            v[u] = q < NV && j >= 0 && j < 2 * nr ? __ldg(xs + j) : 0.0;
+            ex = max(ex, exp_field(v[u]));
+        }
+        ex = (int)__reduce_max_sync(0xffffffffu, (unsigned)ex);
+#pragma unroll
+        for (int u = 0; u < NX; ++u)
+            if (lane + 32 * u < NV) xf[warp][lane + 32 * u] = split29(to_fixed<kFixedBits - 53>(v[u], ex));
+        __syncwarp();
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            long long s1 = 0, s0 = 0;                 // (at most 17 products of 2^58, 34 of 2^57)
+#pragma unroll
+            for (int d = 0; d < W; ++d) {
+                const int2 q = xf[warp][lane + 32 * g + 2 * d];
+                s1 += (long long)a[g][d].x * q.x;
+                s0 += (long long)a[g][d].x * q.y;
+                s0 += (long long)a[g][d].y * q.x;
+            }
+            const unsigned long long lo = ((unsigned long long)s1 << 29) + (unsigned long long)s0;
+            const long long hi = (s1 >> 35) + (s0 >> 63) + (lo < (unsigned long long)s0);
+            double s = ex == 2047 || ea[g] == 2047
+                           ? __hiloint2double(0x7ff80000, 0)
+                           : from_fixed128(hi, lo, ea[g] + ex - 2 * (1022 + kFixedBits) + 29);
+            if (ds.w) {
+                // i f s: the real part's sum goes to the imaginary component, the other back negated
+                s = __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(s), 1),
+                                     __shfl_xor_sync(0xffffffffu, __double2loint(s), 1));
+                if (c == 0) s = __hiloint2double(__double2hiint(s) ^ 0x80000000, __double2loint(s));
+            }
+            if (ds.z) acc[g] = fma(f, s, acc[g]);
+            else if (t == warp) acc[g] = s;
+            else acc[g] += s;
+        }
+        t += tw;
+        if (t >= op.maxt) break;
+        ds = __ldg(desc + t);
+        if (ds.x >= 0) load(ds.y);
+        __syncwarp();                                 // xf is read
+    }
+    if (skip) return;                                 // uniform: written only between launches
+#pragma unroll
+    for (int g = 0; g < G; ++g) part[warp][g][lane] = acc[g];
+    __syncthreads();
+    for (int g = warp; g < G; g += tw) {
+        const int i = i0 + 16 * g;
+        if (i >= nr) continue;
+        double s = part[0][g][lane];
+        for (int q = 1; q < tw; ++q) s += part[q][g][lane];
+        y[2 * ((size_t)l * nr + i) + c] = (probe & 1) ? f2d_fast(d2f_fast(s)) : s;
+    }
+}
+
 bool band_variant_vec_ok(int v, int nr) { return v < 6 || v > 8 || nr % 2 == 0; }
 
 template <typename T, int KB, int V>
 static void band_apply_v(const BandOp<T>& op, const void* x, void* y, const SchedEntry* sched, const Ctrl* ctrl,
                          const Scalings& scaling, int check_broken, cudaStream_t s) {
-    if constexpr (V >= 9) {
-        constexpr int G = V == 9 ? 1 : 2;
+    if constexpr (V >= 11 && sizeof(T) == sizeof(double)) {
+        constexpr int G = V == 11 ? 1 : 2;
+        if (op.fslots) {
+            const int tw = op.maxt < kTermWarps ? (op.maxt < 1 ? 1 : op.maxt) : kTermWarps;
+            dim3 grid((op.nr + 16 * G - 1) / (16 * G), op.nl);
+            launch_pdl(k_band_fixed<KB, G>, grid, dim3(32 * tw), 0, s, op, (const T*)x, (T*)y, sched, ctrl, scaling,
+                       check_broken);
+            return;
+        }
+        band_apply_v<T, KB, 10>(op, x, y, sched, ctrl, scaling, check_broken, s);
+        return;
+    } else if constexpr (V >= 9) {
+        constexpr int G = V == 9 || V == 11 ? 1 : 2;
         if (sizeof(T) == sizeof(double) || op.slots_lo) {
             const int tw = op.maxt < kTermWarps ? (op.maxt < 1 ? 1 : op.maxt) : kTermWarps;
             dim3 grid((op.nr + 16 * G - 1) / (16 * G), op.nl);
@@ -748,6 +889,8 @@ static void band_apply_kb(const BandOp<T>& op, const void* x, void* y, const Sch
         case 8: band_apply_v<T, KB, 8>(op, x, y, sched, ctrl, scaling, check_broken, s); break;
         case 9: band_apply_v<T, KB, 9>(op, x, y, sched, ctrl, scaling, check_broken, s); break;
         case 10: band_apply_v<T, KB, 10>(op, x, y, sched, ctrl, scaling, check_broken, s); break;
+        case 11: band_apply_v<T, KB, sizeof(T) == sizeof(double) ? 11 : 9>(op, x, y, sched, ctrl, scaling, check_broken, s); break;
+        case 12: band_apply_v<T, KB, sizeof(T) == sizeof(double) ? 12 : 10>(op, x, y, sched, ctrl, scaling, check_broken, s); break;
         default: band_apply_v<T, KB, 1>(op, x, y, sched, ctrl, scaling, check_broken, s); break;
     }
 }

@@ -1,4 +1,4 @@
-"""The term-per-warp band kernel (variants 9 and 10) at the edges of its shapes: radial sizes around a
+"""The term-per-warp band kernels (variants 9 and 10; in fixed point 11 and 12) at the edges of its shapes: radial sizes around a
 warp's 16 or 32 elements, every band width, odd sizes, rows of no, one and up to nine terms, real and
 complex bands, several time functions.  Reference: dense numpy in FP64."""
 import numpy as np
@@ -85,3 +85,33 @@ def test_term_per_warp(nl, nr, kb, variant, precision):
     else:
         bound = 2.0 ** -24 * np.sqrt(2) * abs(want) + size * 2.0 ** -40
     assert (abs(got - want) <= bound).all()
+
+
+@pytest.mark.parametrize("nl,nr,kb", SHAPES)
+@pytest.mark.parametrize("variant", [11, 12])
+@pytest.mark.parametrize("scale", [1.0, 1e-290, 1e290])
+def test_fixed_point(nl, nr, kb, variant, scale):
+    """Each factor is rounded to 2^-58 of the largest and the low digits' product dropped (2^-60), each product; the
+    terms' sums round to 2^-53.  (numpy's own sums round as FP64's.)"""
+    got, want, size, peak, terms = _apply(nl, nr, kb, variant, _native.FP64, scale)
+    bound = peak * 3 * 2.0 ** -58 + size * 2.0 ** -53 * (2 * (2 * kb + 1) + 4 * terms + 8)
+    assert (abs(got - want) <= bound).all()
+
+
+@pytest.mark.parametrize("variant", [11, 12])
+def test_fixed_point_nonfinite(variant):
+    """An infinity or a NaN reaches every element whose sum reads it."""
+    import torch
+    nr = 100
+    h = _native.Handle(1, nr, _native.FP64, 4, 0, False, 0)
+    h.set_overlap(1, np.tile([0.0, 1.0], nr))
+    h.add_potential(_native.STORAGE_DIAG, None, 2, np.ones((1, 5 * nr), dtype=np.complex128), False)
+    h.finalize()
+    h.autotune(variant)
+    for bad in (float("inf"), float("nan")):
+        src = torch.ones((1, nr), dtype=torch.complex128, device="cuda")
+        src[0, 50] = complex(bad, 0.0)
+        dst = torch.zeros_like(src)
+        h.matvec(src, dst, 0.0, balanced=False)
+        assert not bool(torch.isfinite(dst.real[0, 48:53]).any())
+        assert bool((dst.real[0, 5:25] == 5.0).all()) and bool((dst.real[0, 75:95] == 5.0).all())
