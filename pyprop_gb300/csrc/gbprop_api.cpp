@@ -113,6 +113,9 @@ struct gbprop_ctx {
     int cgs_part_grid = 0;            // the grid d_cgs_part is sized for
     double* d_cgs_part = nullptr;     // its partial sums
     unsigned* d_gridbar = nullptr;    // its grid-barrier words
+    void* d_cgs_digits = nullptr;     // the fixed-point form's rows and exponents (arnoldi_cgs_digits_bytes)
+    int* d_cgs_exps = nullptr;
+    int cgs_exps_grid = 0;            // the grid d_cgs_exps is sized for
     std::vector<void*> allocs;
 
     // per-phase timing of one un-captured step (gbprop_time_step): when `timing` is set, every
@@ -745,6 +748,20 @@ gbprop_status enqueue_leave(gbprop_ctx* h, void* psi, cudaStream_t s) {
     return GBPROP_OK;
 }
 
+// The fixed-point Gram-Schmidt's buffers for a grid (kept while they are large enough); without memory
+// for them the FP64 form runs.
+void alloc_cgs_digits(gbprop_ctx* h, int grid) {
+    const size_t bytes = arnoldi_cgs_digits_bytes(h->kprec(), h->N, h->m, grid, h->cgs_cache);
+    if (bytes == 0) return;
+    if (grid > h->cgs_exps_grid) {
+        int* p = nullptr;
+        if (h->dalloc(&p, (size_t)kMaxBasis * grid * sizeof(int))) h->d_cgs_digits = nullptr;
+        else h->d_cgs_exps = p, h->cgs_exps_grid = grid;
+    }
+    if (grid <= h->cgs_exps_grid && !h->d_cgs_digits && h->dalloc(&h->d_cgs_digits, bytes)) h->d_cgs_digits = nullptr;
+    cudaGetLastError();
+}
+
 // The Arnoldi part of a step on x (pamp.h:271-400): beta0 = ||x||, m basis vectors, the
 // Hessenberg matrix.  dorth: re-orthogonalisation passes (pamp.h:353-400); brk_tol: the
 // happy-breakdown threshold.
@@ -791,13 +808,14 @@ gbprop_status enqueue_arnoldi(gbprop_ctx* h, int dorth, double brk_tol) {
         // classical Gram-Schmidt against v_0..v_J
         if (fused) {
             GB_LAUNCH(launch_arnoldi_cgs(kp, V, h->d_v0s, N, J, m, h->d_r, h->d_cgs_part, h->d_gridbar, h->d_ctrl,
-                                         h->d_H, J < m - 1, h->cgs_grid, h->cgs_cache, 0, brk_tol, s));
+                                         h->d_H, J < m - 1, h->cgs_grid, h->cgs_cache, 0, brk_tol, h->d_cgs_digits, h->d_cgs_exps, s));
             tick(h, GBPROP_PHASE_GRAM_SCHMIDT);
             continue;
         }
         if (fused_dorth) {
             GB_LAUNCH(launch_arnoldi_cgs(kp, V, nullptr, N, J, m, h->d_r, h->d_cgs_part, h->d_gridbar, h->d_ctrl, h->d_H,
-                                         1, h->cgs_dgrid, h->cgs_cache, 1, brk_tol, s));
+                                         1, h->cgs_dgrid, h->cgs_cache, 1, brk_tol, h->d_cgs_digits,
+                                         h->d_cgs_exps, s));
             tick(h, GBPROP_PHASE_GRAM_SCHMIDT);
             continue;
         }
@@ -1084,6 +1102,9 @@ gbprop_status gbprop_finalize(gbprop_handle h) {
             h->inv_ok = set_inv_chunks(h, 0);
         }
     }
+    // until it is tuned: the form that is quickest or within a tenth of it over 10 x 106 .. 65 x 1500 (FP64:
+    // fixed point; complex64: a warp per term, for long vectors one thread per element)
+    h->band_variant = h->prec == GBPROP_FP64 ? 12 : h->N <= 32768 ? 9 : 4;
     HostBandOp ho = build_band_op(h);
     if (h->prec == GBPROP_FP64) {
         if ((st = upload_band_op<double>(h, ho, &h->t64.op))) return st;
@@ -1129,6 +1150,7 @@ gbprop_status gbprop_finalize(gbprop_handle h) {
             GB_CUDA(cudaMemsetAsync(h->d_gridbar, 0, 64, h->stream));
             (h->double_orth ? h->cgs_dgrid : h->cgs_grid) = grid;
             h->cgs_cache = cache;
+            alloc_cgs_digits(h, grid);
         }
     }
     if ((st = ensure_sched(h, 1024))) return st;
@@ -1445,7 +1467,10 @@ gbprop_status gbprop_autotune(gbprop_handle h, int* variant) {
     if (const char* env_c = std::getenv("GBPROP_SOLVE_CHUNKS")) std::sscanf(env_c, "%d,%d", &pin_c[0], &pin_c[1]);
     const bool pinned = band_variant_available(h, pin_v);
     if (pinned) best = pin_v;
-    for (int v = 0; v < band_variant_count() && !pinned; ++v) {
+    // (complex64 members of a batch: the term-per-warp forms are quicker alone but take more of the SMs'
+    // issue slots, which the other members want; 24 mixed problems 3.97 ms with them, 3.65 without)
+    const int nvar = h->in_batch && kp == 1 ? 9 : band_variant_count();
+    for (int v = 0; v < nvar && !pinned; ++v) {
         if (!band_variant_available(h, v)) continue;
         h->t64.op.variant = v;
         h->t32.op.variant = v;
@@ -2022,6 +2047,7 @@ gbprop_status gbprop_batch_create(gbprop_batch* out, const gbprop_handle* proble
             h->cgs_grid = grid;
             h->cgs_dgrid = 0;
             h->cgs_cache = cache;
+            if (grid > 0) alloc_cgs_digits(h, grid);
         }
         drop_graph(h);
         if (autotune) {

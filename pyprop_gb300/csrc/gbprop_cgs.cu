@@ -90,6 +90,45 @@ __device__ __forceinline__ void cgs_finish(Ctrl* ctrl, double* H, const double* 
     }
 }
 
+// The end of a step with re-orthogonalisation (CTA 0; its warp 0 holds the norms): the column, the
+// counters, the next beta and its breakdown test, as launch_arnoldi_finalize leaves them.
+__device__ __forceinline__ void cgs_finish_dorth(Ctrl* ctrl, double* H, const double* ht, unsigned* bar, unsigned tb,
+                                                 int m, int J, int b, int passes, int again, double pre2, double orig2,
+                                                 double resid2, double brk_tol) {
+    const int nv = J + 1;
+    if (b != 0) return;
+    for (int k = threadIdx.x; k < nv; k += kFuseThreads) {
+        H[2 * ((size_t)k * m + J)] = ht[2 * k];
+        H[2 * ((size_t)k * m + J) + 1] = ht[2 * k + 1];
+        ctrl->h[2 * k] = ht[2 * k];
+        ctrl->h[2 * k + 1] = ht[2 * k + 1];
+    }
+    if (threadIdx.x != 0) return;
+    const double resid = sqrt(resid2);
+    bar[1] = tb;
+    ctrl->nbasis = nv;
+    ctrl->operator_count++;
+    if (J == 0) ctrl->inner_product_count++;
+    // after the third pass the reference counts once more and stops (pamp.h:372-381)
+    ctrl->orthogonalization_count += passes + (again && passes == 3 ? 1 : 0);
+    ctrl->ro_count = passes;
+    ctrl->ro_go = again;
+    ctrl->pre_norm = sqrt(pre2);
+    ctrl->orig_norm = sqrt(orig2);
+    ctrl->resid_norm = resid;
+    if (!isfinite(resid)) ctrl->nonfinite = 1;
+    if (J + 1 >= m) return;
+    if (fabs(resid) < brk_tol) {
+        ctrl->broken = 1;
+        ctrl->breakdown_count++;
+    } else {
+        H[2 * ((size_t)(J + 1) * m + J)] = resid;
+        H[2 * ((size_t)(J + 1) * m + J) + 1] = 0.0;
+        ctrl->beta = resid;
+        set_inv_beta(ctrl, resid);
+    }
+}
+
 // h[0..nvals) = sums over the CTAs' partials (two components per vector and CTA), every CTA the
 // same values: tpv threads per value, a power of two <= 32, so that a value's threads are
 // consecutive lanes of one warp; up to kRound partials per lane and round in fixed point.
@@ -322,37 +361,287 @@ __global__ void __launch_bounds__(kFuseThreads) k_arnoldi_cgs(const double2* __r
         cgs_finish(ctrl, H, hs, m, J, b);
     } else {
         for (int i = tid; i < cl; i += kFuseThreads) w[i0 + i] = ws[i];
-        if (b != 0) return;
-        for (int k = tid; k < nv; k += kFuseThreads) {
-            H[2 * ((size_t)k * m + J)] = ht[2 * k];
-            H[2 * ((size_t)k * m + J) + 1] = ht[2 * k + 1];
-            ctrl->h[2 * k] = ht[2 * k];
-            ctrl->h[2 * k + 1] = ht[2 * k + 1];
+        cgs_finish_dorth(ctrl, H, ht, bar, tb, m, J, b, passes, again, pre2, orig2, resid2, brk_tol);
+    }
+}
+
+// The same step with the products in 56-bit fixed point, for chunks of up to kFixedChunk elements whose
+// basis rows are in shared memory.  A complex product is four FP64 instructions of 64 cycles of a
+// sub-partition, or 12 integer multiply-adds of about 5: every row of V and w is split into two signed
+// 29-bit digits at the largest exponent of the CTA's chunk, and
+//     a x = a1 x1 2^58 + (a1 x0 + a0 x1) 2^29 + a0 x0
+// summed without its last part.  An entry is rounded to 2^-57 of its chunk's largest and a product's
+// dropped part is below 2^-56 of the two chunks' largest, both of either sign; FP64 rounds every partial
+// sum to 2^-53.  A conversion costs what the products of a pair do, so a row is converted once, by the launch that
+// meets it first, and its digits are kept for the step's later ones (Vd, ev: the step's launches share their
+// chunks).  For w - V h the coefficients are brought to one exponent
+// with their rows'.  w itself stays in FP64, an element or two per thread, and the correction is
+// subtracted in FP64.
+constexpr int kFixedOwn = 2;
+constexpr int kFixedChunk = kFixedOwn * kFuseThreads;
+constexpr int kGsBias = 2 * (1075 + 3) - 29;           // exponent of a product of two digits pairs' sums
+
+template <bool DORTH>
+__global__ void __launch_bounds__(kFuseThreads) k_arnoldi_cgs_fixed(const double2* __restrict__ V, long n, int J, int m,
+                                                                    double2* __restrict__ w, double* __restrict__ part,
+                                                                    int4* __restrict__ Vd, int* __restrict__ ev_rows,
+                                                                    unsigned* bar, Ctrl* ctrl, double* H, int update,
+                                                                    int chunk, double brk_tol) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double hs[2 * (kMaxBasis + 1)];
+    __shared__ double ht[DORTH ? 2 * kMaxBasis : 1];   // the column, summed over the passes
+    __shared__ double red[kFuseThreads / 32];
+    __shared__ int2 s_e[kFuseThreads / 32];
+    __shared__ int s_ev[kMaxBasis];                    // the rows' exponents
+    __shared__ int4 s_g[kMaxBasis];                    // the column's digits
+    __shared__ int s_eg, s_again;
+    __shared__ __align__(8) unsigned long long s_bar;
+    const int nv = J + 1, G = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long i0 = (long)b * chunk;
+    const int cl = (int)max(0L, min((long)chunk, n - i0));
+    // shared memory: w chunk | rows of V as digits; w and the newest row as they came and then as digits
+    double2* ws = reinterpret_cast<double2*>(smem_raw);
+    double2* cache = reinterpret_cast<double2*>(smem_raw + (size_t)chunk * sizeof(double2));
+    int4* wd = reinterpret_cast<int4*>(ws);
+    int4* cd = reinterpret_cast<int4*>(cache);
+    // rows of V before the dependency wait, w after it (see k_arnoldi_cgs)
+    const bool tma = cl > 0;
+    const unsigned row = (unsigned)cl * 16;
+    if (tma) {
+        if (tid == 0) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_bar)) : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
-        if (tid != 0) return;
-        const double resid = sqrt(resid2);
-        bar[1] = tb;
-        ctrl->nbasis = nv;
-        ctrl->operator_count++;
-        if (J == 0) ctrl->inner_product_count++;
-        // after the third pass the reference counts once more and stops (pamp.h:372-381)
-        ctrl->orthogonalization_count += passes + (again && passes == 3 ? 1 : 0);
-        ctrl->ro_count = passes;
-        ctrl->ro_go = again;
-        ctrl->pre_norm = sqrt(pre2);
-        ctrl->orig_norm = sqrt(orig2);
-        ctrl->resid_norm = resid;
-        if (!isfinite(resid)) ctrl->nonfinite = 1;
-        if (J + 1 >= m) return;
-        if (fabs(resid) < brk_tol) {
-            ctrl->broken = 1;
-            ctrl->breakdown_count++;
-        } else {
-            H[2 * ((size_t)(J + 1) * m + J)] = resid;
-            H[2 * ((size_t)(J + 1) * m + J) + 1] = 0.0;
-            ctrl->beta = resid;
-            set_inv_beta(ctrl, resid);
+        __syncthreads();
+        if (tid == 0) {
+            asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;"
+                         :: "r"(smem_u32(&s_bar)), "r"(row * (unsigned)nv) : "memory");
+            for (int k = 0; k < J; ++k) bulk_g2s(cd + (size_t)k * chunk, Vd + (size_t)k * n + i0, row, &s_bar);
+            bulk_g2s(cache + (size_t)J * chunk, V + (size_t)J * n + i0, row, &s_bar);
         }
+    }
+    pdl_wait();
+    if (ctrl->broken) {                              // uniform: written only between launches
+        if (tma) {
+            if (tid == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(&s_bar)) : "memory");
+            mbar_wait0(&s_bar);                      // copies in flight land before exit
+        }
+        return;
+    }
+    const bool rnd = ctrl->round_matvec & 2;        // precision probe (FP64 handles)
+    if (tid < J) s_ev[tid] = ev_rows[tid * G + b];
+    unsigned tb = DORTH ? *(volatile const unsigned*)(bar + 1) : (unsigned)J;   // the step's next barrier
+    if (tma) {
+        if (tid == 0) {
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                         :: "r"(smem_u32(&s_bar)), "r"(row) : "memory");
+            bulk_g2s(ws, w + i0, row, &s_bar);
+        }
+        if (!__syncthreads_and(mbar_wait0(&s_bar, wait_budget(ctrl, kInvWaitLimit)))) {
+            if (tid == 0) ctrl->wait_timeout = 1;
+            mbar_wait0(&s_bar);                      // copies in flight land before exit
+            return;
+        }
+    }
+    double2 r[kFixedOwn];                              // this thread's elements of w
+#pragma unroll
+    for (int u = 0; u < kFixedOwn; ++u) {
+        const int i = tid + u * kFuseThreads;
+        r[u] = i < cl ? ws[i] : make_double2(0.0, 0.0);
+    }
+    double orig2 = 0.0, resid2 = 0.0;                  // warp 0: squared norms before and after a pass
+    double pre2 = 0.0;                                 // before the first
+    int passes = 0, again = 0;
+    for (;;) {
+        // ---- digits of w and, in the first pass, of the newest row -----------------------------
+        const bool first = passes == 0;
+        double2 c[kFixedOwn];
+        int ew = 0, ev = 0;
+#pragma unroll
+        for (int u = 0; u < kFixedOwn; ++u) {
+            const int i = tid + u * kFuseThreads;
+            c[u] = first && i < cl ? cache[(size_t)J * chunk + i] : make_double2(0.0, 0.0);
+            ew = max(ew, max(exp_field(r[u].x), exp_field(r[u].y)));
+            ev = max(ev, max(exp_field(c[u].x), exp_field(c[u].y)));
+        }
+        ew = (int)__reduce_max_sync(0xffffffffu, (unsigned)ew);
+        ev = (int)__reduce_max_sync(0xffffffffu, (unsigned)ev);
+        if (lane == 0) s_e[warp] = make_int2(ew, ev);
+        __syncthreads();
+        const int2 em = lane < kFuseThreads / 32 ? s_e[lane] : make_int2(0, 0);
+        ew = (int)__reduce_max_sync(0xffffffffu, (unsigned)em.x);
+        ev = (int)__reduce_max_sync(0xffffffffu, (unsigned)em.y);
+#pragma unroll
+        for (int u = 0; u < kFixedOwn; ++u) {
+            const int i = tid + u * kFuseThreads;
+            if (i >= cl) break;
+            const int2 x = split29(to_fixed<3>(r[u].x, ew)), y = split29(to_fixed<3>(r[u].y, ew));
+            wd[i] = make_int4(x.x, x.y, y.x, y.y);
+            if (!first) continue;
+            const int2 p = split29(to_fixed<3>(c[u].x, ev)), q = split29(to_fixed<3>(c[u].y, ev));
+            const int4 v = make_int4(p.x, p.y, q.x, q.y);
+            cd[(size_t)J * chunk + i] = v;
+            Vd[(size_t)J * n + i0 + i] = v;
+        }
+        if (first && tid == 0) s_ev[J] = ev_rows[J * G + b] = ev;
+        __syncthreads();
+        // ---- phase A: partial inner products, one warp per basis vector --------------------------
+        for (int k = warp; k < nv; k += kFuseThreads / 32) {
+            const int4* dk = cd + (size_t)k * chunk;
+            const int ek = s_ev[k];
+            // (at most 2 kFixedChunk / 32 products of 2^54, twice as many of 2^55)
+            long long r1 = 0, r0 = 0, i1 = 0, i0s = 0;
+            auto add = [&](const int4 v, const int4 x) {
+                mad_wide(r1, v.x, x.x);
+                mad_wide(r0, v.x, x.y);
+                mad_wide(r0, v.y, x.x);
+                mad_wide(r1, v.z, x.z);
+                mad_wide(r0, v.z, x.w);
+                mad_wide(r0, v.w, x.z);
+                const int a = -v.z, c = -v.w;
+                mad_wide(i1, v.x, x.z);
+                mad_wide(i0s, v.x, x.w);
+                mad_wide(i0s, v.y, x.z);
+                mad_wide(i1, a, x.x);
+                mad_wide(i0s, a, x.y);
+                mad_wide(i0s, c, x.x);
+            };
+#pragma unroll 4
+            for (int i = lane; i < cl; i += 32) add(dk[i], wd[i]);
+            const bool bad = ek == 2047 || ew == 2047;
+            const double nan = __hiloint2double(0x7ff80000, 0);
+            const double ar = warp_fixed_sum(bad ? nan : from_digits(r1, r0, ek + ew - kGsBias));
+            const double ai = warp_fixed_sum(bad ? nan : from_digits(i1, i0s, ek + ew - kGsBias));
+            if (lane == 0) {
+                part[((size_t)k * G + b) * 2] = ar;
+                part[((size_t)k * G + b) * 2 + 1] = ai;
+            }
+        }
+        if (DORTH && passes == 0) {
+            // ||w||^2 before the first pass, as one more vector's partial
+            double t = 0.0;
+#pragma unroll
+            for (int u = 0; u < kFixedOwn; ++u) t = fma(r[u].y, r[u].y, fma(r[u].x, r[u].x, t));
+            t = warp_fixed_sum(t);
+            if (lane == 0) red[warp] = t;
+            __syncthreads();
+            if (warp == 0) {
+                t = warp_fixed_sum(lane < kFuseThreads / 32 ? red[lane] : 0.0);
+                if (lane == 0) {
+                    part[((size_t)nv * G + b) * 2] = t;
+                    part[((size_t)nv * G + b) * 2 + 1] = 0.0;
+                }
+            }
+        }
+        if (!grid_barrier(bar, G, tb++, ctrl)) return;
+
+        // ---- phase B: h = sum of the partials -----------------------------------------------
+        cgs_sum_partials(part, G, 2 * nv + (DORTH && passes == 0 ? 1 : 0), hs);
+        __syncthreads();
+        if (DORTH) {
+            if (passes == 0) pre2 = orig2 = hs[2 * nv];
+            for (int k = tid; k < 2 * nv; k += kFuseThreads) ht[k] = passes ? ht[k] + hs[k] : hs[k];
+        }
+        if (update) {
+            // the column's digits, every h_k 2^(row exponent) at the largest's exponent
+            if (warp == 0) {
+                int e[2], ek[2], eg = 0;
+                bool bad = false;
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int k = lane + 32 * u;
+                    const bool on = k < nv;
+                    e[u] = on ? max(exp_field(hs[2 * k]), exp_field(hs[2 * k + 1])) : 0;
+                    const int v = on ? s_ev[k] : 0;
+                    bad |= e[u] == 2047 || v == 2047;
+                    ek[u] = e[u] && v ? e[u] + v : 0;
+                    eg = max(eg, ek[u]);
+                }
+                eg = (int)__reduce_max_sync(0xffffffffu, (unsigned)eg);
+                bad = __any_sync(0xffffffffu, bad);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int k = lane + 32 * u;
+                    if (k >= nv) continue;
+                    const int sh = ek[u] ? min(eg - ek[u], 60) : 60;
+                    auto digits = [&](double h) {
+                        const long long f = to_fixed<3>(h, e[u]);
+                        return split29(sh ? (f + (1ll << (sh - 1))) >> sh : f);
+                    };
+                    const int2 x = digits(hs[2 * k]), y = digits(hs[2 * k + 1]);
+                    s_g[k] = make_int4(x.x, x.y, y.x, y.y);
+                }
+                if (lane == 0) s_eg = bad ? -1 : eg;
+            }
+            __syncthreads();
+            const int eg = s_eg;
+            double nrm = 0.0;
+#pragma unroll
+            for (int u = 0; u < kFixedOwn; ++u) {
+                const int i = tid + u * kFuseThreads;
+                if (i >= cl) break;
+                // (at most 2 kMaxBasis products of 2^54, twice as many of 2^55)
+                long long r1 = 0, r0 = 0, i1 = 0, i0s = 0;
+#pragma unroll 4
+                for (int k = 0; k < nv; ++k) {
+                    const int4 v = cd[(size_t)k * chunk + i], g = s_g[k];
+                    const int a = -v.z, c = -v.w;
+                    mad_wide(r1, v.x, g.x);
+                    mad_wide(r0, v.x, g.y);
+                    mad_wide(r0, v.y, g.x);
+                    mad_wide(r1, a, g.z);
+                    mad_wide(r0, a, g.w);
+                    mad_wide(r0, c, g.z);
+                    mad_wide(i1, v.x, g.z);
+                    mad_wide(i0s, v.x, g.w);
+                    mad_wide(i0s, v.y, g.z);
+                    mad_wide(i1, v.z, g.x);
+                    mad_wide(i0s, v.z, g.y);
+                    mad_wide(i0s, v.w, g.x);
+                }
+                if (eg < 0) {
+                    r[u] = make_double2(__hiloint2double(0x7ff80000, 0), __hiloint2double(0x7ff80000, 0));
+                } else {
+                    r[u].x -= from_digits(r1, r0, eg - kGsBias);
+                    r[u].y -= from_digits(i1, i0s, eg - kGsBias);
+                }
+                if (rnd) r[u] = make_double2(f2d_fast(d2f_fast(r[u].x)), f2d_fast(d2f_fast(r[u].y)));
+                if (!DORTH) w[i0 + i] = r[u];
+                nrm = fma(r[u].x, r[u].x, nrm);
+                nrm = fma(r[u].y, r[u].y, nrm);
+            }
+            nrm = warp_fixed_sum(nrm);
+            if (lane == 0) red[warp] = nrm;
+            __syncthreads();
+            if (warp == 0) {
+                const double t = warp_fixed_sum(lane < kFuseThreads / 32 ? red[lane] : 0.0);
+                // (without DORTH: for the next solve's beta)
+                if (lane == 0) part[(size_t)(DORTH ? nv + 1 : nv) * G * 2 + b] = t;
+            }
+        }
+        if (!DORTH) break;
+        if (!grid_barrier(bar, G, tb++, ctrl)) return;
+        if (warp == 0) {
+            const double t = warp_fixed_sum_of(part + (size_t)(nv + 1) * G * 2, G, 1);
+            if (passes > 0) orig2 = resid2;
+            resid2 = t;
+            if (lane == 0) s_again = t < 0.717 * 0.717 * orig2;      // pamp.h:369
+        }
+        __syncthreads();
+        again = s_again;
+        // the reference loop runs at most MaxOrthogonalizationCount = 3 passes (pamp.h:75,375)
+        if (!again || passes == 3) break;
+        ++passes;
+    }
+    if constexpr (!DORTH) {
+        cgs_finish(ctrl, H, hs, m, J, b);
+    } else {
+#pragma unroll
+        for (int u = 0; u < kFixedOwn; ++u) {
+            const int i = tid + u * kFuseThreads;
+            if (i < cl) w[i0 + i] = r[u];
+        }
+        cgs_finish_dorth(ctrl, H, ht, bar, tb, m, J, b, passes, again, pre2, orig2, resid2, brk_tol);
     }
 }
 
@@ -616,6 +905,16 @@ size_t arnoldi_cgs_smem(int prec, long n, int nv, int grid, int with_v0, int cac
     return b;
 }
 
+static int cgs_chunk(long n, int grid) { return (int)(((n + grid - 1) / grid + 7) / 8 * 8); }
+
+// Fixed point wherever the rows are in shared memory and a thread holds its elements of w (up to 1024 a CTA: all
+// but long vectors of small bases).
+static bool cgs_fixed(int cache, int chunk) { return cache && chunk <= kFixedChunk; }
+
+static decltype(&k_arnoldi_cgs_fixed<false>) cgs_kernel_fixed(int dorth) {
+    return dorth ? k_arnoldi_cgs_fixed<true> : k_arnoldi_cgs_fixed<false>;
+}
+
 static decltype(&k_arnoldi_cgs<true, false>) cgs_kernel64(int cache, int dorth) {
     return dorth ? (cache ? k_arnoldi_cgs<true, true> : k_arnoldi_cgs<false, true>)
                  : (cache ? k_arnoldi_cgs<true, false> : k_arnoldi_cgs<false, false>);
@@ -642,11 +941,14 @@ static cudaError_t cgs_coop_launch(Kern kern, int grid, size_t smem, cudaStream_
 
 cudaError_t launch_arnoldi_cgs(int prec, const void* V, const void* v0, long n, int J, int m, void* w,
                                double* part, unsigned* bar, Ctrl* ctrl, double* H, int update, int grid, int cache,
-                               int dorth, double brk_tol, cudaStream_t s) {
+                               int dorth, double brk_tol, void* Vd, int* ev_rows, cudaStream_t s) {
     count_launch();
-    const int chunk = (int)(((n + grid - 1) / grid + 7) / 8 * 8);
+    const int chunk = cgs_chunk(n, grid);
     const size_t smem = arnoldi_cgs_smem(prec, n, J + 1, grid, v0 != nullptr, cache);
     if (prec == 0) {
+        if (Vd && cgs_fixed(cache, chunk))
+            return cgs_coop_launch(cgs_kernel_fixed(dorth), grid, smem, s, (const double2*)V, n, J, m, (double2*)w, part, (int4*)Vd,
+                                   ev_rows, bar, ctrl, H, update, chunk, brk_tol);
         auto kern = cgs_kernel64(cache, dorth);
         return cgs_coop_launch(kern, grid, smem, s, (const double2*)V, n, J, m, (double2*)w, part, bar, ctrl, H, update,
                                chunk, brk_tol);
@@ -655,6 +957,24 @@ cudaError_t launch_arnoldi_cgs(int prec, const void* V, const void* v0, long n, 
     auto kern = cache ? k_arnoldi_cgs32<true> : k_arnoldi_cgs32<false>;
     return cgs_coop_launch(kern, grid, smem, s, (const float2*)V, (const float4*)v0, n, J, m, (float2*)w,
                            (float4*)part, bar, ctrl, H, update, chunk);
+}
+
+size_t arnoldi_cgs_digits_bytes(int prec, long n, int m, int grid, int cache) {
+    return prec == 0 && cgs_fixed(cache, cgs_chunk(n, grid)) ? (size_t)m * n * sizeof(int4) : 0;
+}
+
+// resident CTAs per SM of the FP64 form (of both where it may be the fixed-point one)
+static cudaError_t cgs_occupancy64(long n, int grid, int cache, int dorth, size_t smem, int* per_sm) {
+    auto kern = cgs_kernel64(cache, dorth);
+    allow_max_smem(kern);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, kFuseThreads, smem);
+    if (e == cudaSuccess && cgs_fixed(cache, cgs_chunk(n, grid))) {
+        int fixed = 0;
+        allow_max_smem(cgs_kernel_fixed(dorth));
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fixed, cgs_kernel_fixed(dorth), kFuseThreads, smem);
+        *per_sm = std::min(*per_sm, fixed);
+    }
+    return e;
 }
 
 // Grid of co-resident CTAs for this configuration: one CTA per SM, or one per 32 elements where
@@ -673,9 +993,7 @@ int arnoldi_cgs_grid(int prec, long n, int m, int with_v0, int cache, int dorth)
     int per_sm = 0;
     cudaError_t e;
     if (prec == 0) {
-        auto kern = cgs_kernel64(cache, dorth);
-        allow_max_smem(kern);
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFuseThreads, smem);
+        e = cgs_occupancy64(n, grid, cache, dorth, smem, &per_sm);
     } else {
         auto kern = cache ? k_arnoldi_cgs32<true> : k_arnoldi_cgs32<false>;
         allow_max_smem(kern);
@@ -707,9 +1025,7 @@ int arnoldi_cgs_grid_batch(int prec, long n, int m, int with_v0, int* cache) {
         int per_sm = 0;
         cudaError_t e;
         if (prec == 0) {
-            auto kern = cgs_kernel64(c, 0);
-            allow_max_smem(kern);
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFuseThreads, smem);
+            e = cgs_occupancy64(n, grid, c, 0, smem, &per_sm);
         } else {
             auto kern = c ? k_arnoldi_cgs32<true> : k_arnoldi_cgs32<false>;
             allow_max_smem(kern);

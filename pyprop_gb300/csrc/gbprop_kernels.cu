@@ -682,18 +682,13 @@ __global__ void __launch_bounds__(32 * kTermWarps) k_band_split(BandOp<T> op, co
 
 // The same split in 58-bit fixed point (variants 11 and 12: 1 or 2 groups of 16 elements per warp).
 // A product of FP64 numbers is one FP64 instruction, 64 cycles of its sub-partition, but three
-// integer multiply-adds of 2 each: with a = a1 2^29 + a0 and x = x1 2^29 + x0 in signed digits,
+// integer multiply-adds of about 5 each: with a = a1 2^29 + a0 and x = x1 2^29 + x0 in signed digits,
 //     a x = a1 x1 2^58 + (a1 x0 + a0 x1) 2^29 + a0 x0,
 // the last of which, 2^-60 of the largest product, is left out.  Coefficients are at the exponent of their
 // row's largest, x at that of the largest entry a warp reads (16 G + 2 KB elements), so a row errs by
 // 2^-58 of the largest coefficient times the largest entry and each product, where FP64 rounds every
 // partial sum to 2^-53.
 constexpr int kFixedBits = 58;
-__device__ __forceinline__ int2 split29(long long f) {
-    const int lo = ((int)(unsigned)f << 3) >> 3;
-    return make_int2((int)((f - lo) >> 29), lo);
-}
-
 __global__ void k_band_fixed_slots(const double* __restrict__ slots, int nr, int width, int2* __restrict__ digits,
                                    int* __restrict__ exps) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -772,15 +767,12 @@ __global__ void __launch_bounds__(32 * kTermWarps) k_band_fixed(BandOp<double> o
 #pragma unroll
             for (int d = 0; d < W; ++d) {
                 const int2 q = xf[warp][lane + 32 * g + 2 * d];
-                s1 += (long long)a[g][d].x * q.x;
-                s0 += (long long)a[g][d].x * q.y;
-                s0 += (long long)a[g][d].y * q.x;
+                mad_wide(s1, a[g][d].x, q.x);
+                mad_wide(s0, a[g][d].x, q.y);
+                mad_wide(s0, a[g][d].y, q.x);
             }
-            const unsigned long long lo = ((unsigned long long)s1 << 29) + (unsigned long long)s0;
-            const long long hi = (s1 >> 35) + (s0 >> 63) + (lo < (unsigned long long)s0);
-            double s = ex == 2047 || ea[g] == 2047
-                           ? __hiloint2double(0x7ff80000, 0)
-                           : from_fixed128(hi, lo, ea[g] + ex - 2 * (1022 + kFixedBits) + 29);
+            double s = ex == 2047 || ea[g] == 2047 ? __hiloint2double(0x7ff80000, 0)
+                                                   : from_digits(s1, s0, ea[g] + ex - 2 * (1022 + kFixedBits) + 29);
             if (ds.w) {
                 // i f s: the real part's sum goes to the imaginary component, the other back negated
                 s = __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(s), 1),
