@@ -250,12 +250,13 @@ gbprop_status gbprop_expokit_advance(gbprop_handle h, void* psi, int nsteps, con
                                      double dt_re, double dt_im, double tol, double anorm,
                                      gbprop_expokit_stats* stats);
 
-/* Band-kernel tile autotuner: times every tile shape of the TensorPotential matvec
- * kernel on this handle's operator and keeps the fastest; *variant (if not NULL)
- * receives its index.  Synchronises the handle's stream.  If *variant >= 0 on entry,
- * that shape is selected without timing (GBPROP_EINVAL if it does not exist, or if it
- * does not apply: shapes 6, 7 and 8 form two radial elements per thread and need an even
- * radial size).  No counterpart in the reference (its generated kernels have one shape). */
+/* Autotuner: times the forms of the TensorPotential matvec kernel that can be the quickest on
+ * this handle's operator (FP64 9 to 12, FP32-mixed 4 to 10, in a batch 4 to 8) and keeps the
+ * fastest; *variant (if not NULL) receives its index.  Likewise the shapes of the
+ * overlap-factor solves, outside a batch.  Synchronises the handle's stream.  If *variant >= 0 on
+ * entry, that form is selected without timing (GBPROP_EINVAL if it does not exist, or if it
+ * does not apply: 6, 7 and 8 form two radial elements per thread and need an even radial
+ * size, 11 and 12 multiply in fixed point and are FP64's).  No counterpart in the reference (its generated kernels have one shape). */
 gbprop_status gbprop_autotune(gbprop_handle h, int* variant);
 
 /* Field-free bound states: for every angular row l the eigenpairs with E < emax of the

@@ -1470,7 +1470,9 @@ gbprop_status gbprop_autotune(gbprop_handle h, int* variant) {
     // (complex64 members of a batch: the term-per-warp forms are quicker alone but take more of the SMs'
     // issue slots, which the other members want; 24 mixed problems 3.97 ms with them, 3.65 without)
     const int nvar = h->in_batch && kp == 1 ? 9 : band_variant_count();
-    for (int v = 0; v < nvar && !pinned; ++v) {
+    // (the forms before are never the quickest over 10 x 106 .. 65 x 1500: FP64 12.8 us and more at 10 x 106
+    // against 6, 18 and more at 64 x 1000 against 12.6; the staged tiles of complex64 behind variant 4)
+    for (int v = kp == 0 ? 9 : 4; v < nvar && !pinned; ++v) {
         if (!band_variant_available(h, v)) continue;
         h->t64.op.variant = v;
         h->t32.op.variant = v;
