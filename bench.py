@@ -42,13 +42,13 @@ FP32_PEAK_TFLOPS = 69.9
 # capture each comes from is named in PHASE_TRAFFIC_SOURCE)
 PHASE_TRAFFIC = {
     ("fp64", "band"): 20802560, ("fp32-mixed", "band"): 20300288,
-    ("fp64", "solve"): 1408256, ("fp32-mixed", "solve"): 826000,
-    ("fp64", "gram_schmidt"): 16416768, ("fp32-mixed", "gram_schmidt"): 8750336,
+    ("fp64", "solve"): 1678336, ("fp32-mixed", "solve"): 826000,
+    ("fp64", "gram_schmidt"): 16450304, ("fp32-mixed", "gram_schmidt"): 8750336,
 }
 PHASE_TRAFFIC_SOURCE = {
     "band": "profiles/band_kernel_hydrogen_large.md (ncu, dram__bytes_read/write.sum, one launch)",
-    "solve": "profiles/k_solve_inv_fp64_hydrogen_large.md, profiles/k_solve_mixed_hydrogen_large.md "
-             "(ncu --set full, one launch; the inverse band and the factor stay in L2)",
+    "solve": "profiles/k_solve_rows_hydrogen_large.md (ncu --set full, one launch; the inverse band and the factor "
+             "stay in L2)",
     "gram_schmidt": "profiles/k_arnoldi_cgs_hydrogen_large.md, profiles/k_arnoldi_cgs32_hydrogen_large.md "
                     "(ncu --set full, Arnoldi step J = 14)",
 }
@@ -807,10 +807,12 @@ def measure_single(args, precision, device, world, with_e2e=True):
         compute = {"unit": "TFLOP/s", "achieved": band_flops / (t_band * 1e-3) / 1e12, "peak": FP32_PEAK_TFLOPS,
                    "peak_source": "measured FP32 FMA issue rate on GB300", "what": "FP32 ops of the compensated sums"}
     compute["frac"] = compute["achieved"] / compute["peak"]
-    kernels = {"solve": "k_solve_inv (overlap-factor solves U^-1, U^-T)" if precision == "fp64" else
-               "k_solve_mixed / k_solve_inv (complex64 basis solves, FP64 state solve)",
-               "band": "k_band_apply (TensorPotentialMultiply, all terms)",
-               "gram_schmidt": "k_arnoldi_cgs (cooperative Gram-Schmidt) + k_norm",
+    kernels = {"solve": "k_solve_rows (overlap-factor solves U^-1, U^-T)" if precision == "fp64" else
+               "k_solve_rows (complex64 basis solves, FP64 state solve)",
+               "band": "k_band_fixed (TensorPotentialMultiply, all terms)" if precision == "fp64" else
+               "k_band_apply (TensorPotentialMultiply, all terms)",
+               "gram_schmidt": "k_arnoldi_cgs_fixed (cooperative Gram-Schmidt) + k_norm" if precision == "fp64" else
+               "k_arnoldi_cgs32 (cooperative Gram-Schmidt) + k_norm",
                "exponential": "k_expm_cluster (Pade scaling-and-squaring)",
                "combine": "k_combine", "other": "k_tbmv + step bookkeeping"}
     tp = per_phase[top]
