@@ -536,11 +536,13 @@ gbprop_status upload_band_op(gbprop_ctx* h, const HostBandOp& ho, BandOp<T>* out
         const int W = 2 * ho.kb + 1, nslots = (int)(ho.slots.size() / ((size_t)W * h->nr));
         int2* fs;
         int* fe;
-        if ((st = h->dalloc(&fs, ho.slots.size() * sizeof(int2)))) return st;
-        if ((st = h->dalloc(&fe, (size_t)nslots * h->nr * sizeof(int)))) return st;
-        GB_CUDA(launch_band_fixed_slots((const double*)slots, nslots, h->nr, W, fs, fe, h->stream));
-        out->fslots = fs;
-        out->fexp = fe;
+        // (without memory for them the FP64 forms remain)
+        if (!h->dalloc(&fe, (size_t)nslots * h->nr * sizeof(int)) && !h->dalloc(&fs, ho.slots.size() * sizeof(int2))) {
+            GB_CUDA(launch_band_fixed_slots((const double*)slots, nslots, h->nr, W, fs, fe, h->stream));
+            out->fslots = fs;
+            out->fexp = fe;
+        }
+        cudaGetLastError();
     }
     if (sizeof(T) < sizeof(double)) {
         // complex64 path: the rounding remainder of every coefficient, so the operator
