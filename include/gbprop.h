@@ -251,12 +251,16 @@ gbprop_status gbprop_expokit_advance(gbprop_handle h, void* psi, int nsteps, con
                                      gbprop_expokit_stats* stats);
 
 /* Autotuner: times the forms of the TensorPotential matvec kernel that can be the quickest on
- * this handle's operator (FP64 9 to 12, FP32-mixed 4 to 10, in a batch 4 to 8) and keeps the
+ * this handle's operator (FP64 9 and 10, FP32-mixed 4 to 10, in a batch 4 to 8) and keeps the
  * fastest; *variant (if not NULL) receives its index.  Likewise the shapes of the
  * overlap-factor solves, outside a batch.  Synchronises the handle's stream.  If *variant >= 0 on
  * entry, that form is selected without timing (GBPROP_EINVAL if it does not exist, or if it
  * does not apply: 6, 7 and 8 form two radial elements per thread and need an even radial
- * size, 11 and 12 multiply in fixed point and are FP64's).  No counterpart in the reference (its generated kernels have one shape). */
+ * size, 11 and 12 are FP64's).  11 and 12 multiply in 58-bit fixed point, up to a quarter
+ * quicker: an output then errs by 2^-58 of its row's largest coefficient times the largest of the
+ * 28 or 44 input elements around it, where the other forms err by 2^-53 of the element's own
+ * sum of |a| |x|; their digits take as much device memory as the operator, from the first
+ * time they are asked for.  No counterpart in the reference (its generated kernels have one shape). */
 gbprop_status gbprop_autotune(gbprop_handle h, int* variant);
 
 /* Field-free bound states: for every angular row l the eigenpairs with E < emax of the

@@ -532,18 +532,7 @@ gbprop_status upload_band_op(gbprop_ctx* h, const HostBandOp& ho, BandOp<T>* out
     out->desc = dd;
     out->fslots = nullptr;
     out->fexp = nullptr;
-    if (sizeof(T) == sizeof(double) && !ho.slots.empty()) {
-        const int W = 2 * ho.kb + 1, nslots = (int)(ho.slots.size() / ((size_t)W * h->nr));
-        int2* fs;
-        int* fe;
-        // (without memory for them the FP64 forms remain)
-        if (!h->dalloc(&fe, (size_t)nslots * h->nr * sizeof(int)) && !h->dalloc(&fs, ho.slots.size() * sizeof(int2))) {
-            GB_CUDA(launch_band_fixed_slots((const double*)slots, nslots, h->nr, W, fs, fe, h->stream));
-            out->fslots = fs;
-            out->fexp = fe;
-        }
-        cudaGetLastError();
-    }
+    out->nslots = (int)(ho.slots.size() / ((size_t)(2 * ho.kb + 1) * h->nr));
     if (sizeof(T) < sizeof(double)) {
         // complex64 path: the rounding remainder of every coefficient, so the operator
         // applied is the FP64 one (to ~2^-48) and only the FP32 sums round
@@ -1104,9 +1093,10 @@ gbprop_status gbprop_finalize(gbprop_handle h) {
             h->inv_ok = set_inv_chunks(h, 0);
         }
     }
-    // until it is tuned: the form that is quickest or within a tenth of it over 10 x 106 .. 65 x 1500 (FP64:
-    // fixed point; complex64: a warp per term, for long vectors one thread per element)
-    h->band_variant = h->prec == GBPROP_FP64 ? 12 : h->N <= 32768 ? 9 : 4;
+    // until it is tuned: the form that is quickest or within a sixth of it over 4 x 60 .. 65 x 1500: a warp per
+    // term, for long complex64 vectors one thread per element (37 x 811: 9.0 us against 9.3; 64 x 1000: 13.0
+    // against 10.9, the best 9.8)
+    h->band_variant = h->prec == GBPROP_FP64 || h->N <= 32768 ? 9 : 4;
     HostBandOp ho = build_band_op(h);
     if (h->prec == GBPROP_FP64) {
         if ((st = upload_band_op<double>(h, ho, &h->t64.op))) return st;
@@ -1437,11 +1427,26 @@ gbprop_status gbprop_tensor_multiply_bandnh(int storage, const void* V, int npai
     return GBPROP_OK;
 }
 
-// Variants 6, 7 and 8 (two elements per thread, vector loads) need an even radial size.
-bool band_variant_available(const gbprop_ctx* h, int v) {
+// Variants 6, 7 and 8 (two elements per thread, vector loads) need an even radial size; 11 and 12 take the
+// coefficients' digits, formed when one of them is first asked for.
+bool band_variant_available(gbprop_ctx* h, int v) {
     if (v < 0 || v >= band_variant_count()) return false;
     if (v < 6) return true;
-    if (v >= 11) return h->kprec() == 0 && h->t64.op.fslots != nullptr;
+    if (v >= kBandFixed) {
+        BandOp<double>& op = h->t64.op;
+        if (h->kprec() != 0 || op.nslots == 0) return false;
+        if (op.fslots) return true;
+        const size_t rows = (size_t)op.nslots * op.nr, W = 2 * op.kb + 1;
+        int2* fs;
+        int* fe;
+        const bool ok = !h->dalloc(&fe, rows * sizeof(int)) && !h->dalloc(&fs, rows * W * sizeof(int2)) &&
+                        launch_band_fixed_slots(op.slots, op.nslots, op.nr, (int)W, fs, fe, h->stream) == cudaSuccess;
+        cudaGetLastError();
+        if (!ok) return false;
+        op.fslots = fs;
+        op.fexp = fe;
+        return true;
+    }
     if (!band_variant_vec_ok(v, h->nr)) return false;
     return h->kprec() == 0 || h->t32.op.slots_lo != nullptr;
 }
@@ -1470,10 +1475,12 @@ gbprop_status gbprop_autotune(gbprop_handle h, int* variant) {
     const bool pinned = band_variant_available(h, pin_v);
     if (pinned) best = pin_v;
     // (complex64 members of a batch: the term-per-warp forms are quicker alone but take more of the SMs'
-    // issue slots, which the other members want; 24 mixed problems 3.97 ms with them, 3.65 without)
-    const int nvar = h->in_batch && kp == 1 ? 9 : band_variant_count();
-    // (the forms before are never the quickest over 10 x 106 .. 65 x 1500: FP64 12.8 us and more at 10 x 106
-    // against 6, 18 and more at 64 x 1000 against 12.6; the staged tiles of complex64 behind variant 4)
+    // issue slots, which the other members want; 24 mixed problems 3.97 ms with them, 3.57 without.  The
+    // fixed-point forms are for callers that ask for them: timing must not choose a handle's accuracy)
+    const int nvar = h->in_batch && kp == 1 ? 9 : kBandFixed;
+    // (the forms before are never the quickest over 10 x 106 .. 65 x 1500, an application with its launch: FP64
+    // 13 us and more at 10 x 106 against 5.1, 17.8 against 17.3 at 64 x 1000, 24.1 against 23.0 at 65 x 1500; the
+    // staged tiles of complex64 are behind variant 4.  They are there to be asked for.)
     for (int v = kp == 0 ? 9 : 4; v < nvar && !pinned; ++v) {
         if (!band_variant_available(h, v)) continue;
         h->t64.op.variant = v;

@@ -136,7 +136,9 @@ template <typename T> struct BandOp {
     // where the factor is i instead of 1
     int maxt;
     const int4* desc;
-    // FP64: the slots as 58-bit fixed-point numbers (see split29) at each row's largest exponent
+    // FP64, variants 11 and 12 only (else null): the slots as 58-bit fixed-point numbers (see split29) at each
+    // row's largest exponent
+    int nslots;
     const int2* fslots;
     const int* fexp;         // nslots x nr
 };
@@ -302,6 +304,7 @@ cudaError_t launch_zero(void* p, size_t bytes, cudaStream_t s);
 
 int grid_reduce_blocks();
 int band_variant_count();
+constexpr int kBandFixed = 11;               // the first of the fixed-point forms
 // fixed-point form of FP64 slots (nslots x (2 kb + 1) x nr) and the row exponents (nslots x nr)
 cudaError_t launch_band_fixed_slots(const double* slots, int nslots, int nr, int width, int2* digits, int* exps,
                                     cudaStream_t s);

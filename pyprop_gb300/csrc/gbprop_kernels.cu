@@ -154,7 +154,9 @@ __device__ void block_partials<16>(double (&acc)[16], int nvalid, double* partia
 // (threads per block, radial elements per thread).
 // Variants 4 and 5 stage nothing: one thread per element reads its stencil through L1.
 // Variants 6, 7, 8 (even nr): two elements per thread with vector loads (k_band_apply_x2 / _x2d;
-// 128, 64, 32 threads).  Variants 9, 10: a lane per component, a warp per term (k_band_split).
+// 128, 64, 32 threads).  Variants 9, 10: a lane per component, a warp per term (k_band_split); 11, 12: that in
+// fixed point (k_band_fixed, FP64 handles).  The autotuner times 9 and 10 of FP64 handles and 4 to 10 of
+// complex64 ones; the others run where a caller asks for them.
 constexpr int kBandVariants = 13;
 __host__ __device__ constexpr int band_threads(int v) {
     return v == 0 ? 64 : v == 1 ? 128 : v == 2 ? 128 : v == 3 ? 256 : v == 4 ? 128 : 256;
@@ -573,9 +575,10 @@ __global__ void __launch_bounds__(THREADS) k_band_apply_x2d(BandOp<double> op, c
 // counts is how evenly the warp instructions fall on the 608 sub-partitions: against one thread per
 // element or pair of elements that walks through its row's terms this has six times as many warps of a
 // sixth of the length, and their loads are in flight together instead of term after term.  A warp's
-// descriptor is one 16-byte load; nothing depends on the row table.  Measured per application, best of the
-// other forms and this: FP64 10 x 106 11.8 -> 5.9 us, 23 x 437 13.7 -> 6.6, 64 x 1000 18.0 -> 17.0;
-// complex64 10 x 106 7.8 -> 5.8, 64 x 1000 10.1 -> 13.0 (there the two-element form stays the better).
+// descriptor is one 16-byte load; nothing depends on the row table.  Measured per application with its launch, best
+// of the other forms and this: FP64 10 x 106 13.0 -> 5.1 us, 23 x 437 13.4 -> 6.4, 64 x 1000 17.8 -> 17.3, 65 x 1500
+// 24.1 -> 23.0; complex64 10 x 106 8.1 -> 5.1, 64 x 1000 9.8 -> 12.7 (there the two-element form stays the better).
+// One group of 16 elements is the quicker for FP64 everywhere, by up to a sixth (37 x 811: 11.1 us against 13.0).
 constexpr int kTermWarps = 4;
 template <typename T, int KB, int G>
 __global__ void __launch_bounds__(32 * kTermWarps) k_band_split(BandOp<T> op, const T* __restrict__ x,
@@ -688,10 +691,15 @@ __global__ void __launch_bounds__(32 * kTermWarps) k_band_split(BandOp<T> op, co
 //     a x = a1 x1 2^58 + (a1 x0 + a0 x1) 2^29 + a0 x0,
 // the last of which, 2^-60 of the largest product, is left out.  Coefficients are at the exponent of their
 // row's largest, x at that of the largest entry a warp reads (16 G + 2 KB elements), so a row errs by
-// 2^-58 of the largest coefficient times the largest entry and each product, where FP64 rounds every
-// partial sum to 2^-53.  Measured per application, FP64 products and these: 64 x 1000 17.0 -> 12.6 us
-// (1.6 TB/s of coefficients, from L2), 65 x 1500 24.8 -> 17.5, 23 x 437 6.6 -> 5.8, 10 x 106 6.0 -> 6.1; relative L2
-// error against 64 bits the same (5e-16 to 2e-15).
+// 2^-58 of the largest coefficient times the largest entry and each product.  That is a bound for the window and
+// not, as FP64's, for the element: beside entries 2^30 times its size an entry keeps 28 of its 53 bits.  States fall
+// that steeply towards the origin and in their tails (in a 64 x 1000 step two thirds of the warps' windows hold
+// an element whose sum of |a| |x| is 2^8 below the largest product, half of them one 2^16 below), and a relaxation
+// of 16 x 300 errs by 2.1e-15 against 1.9e-15.  So neither the default nor the autotuner takes these forms; a caller to whom the L2 error
+// counts asks for them (gbprop_autotune, GBPROP_BAND_VARIANT).  An infinity or NaN makes NaN of all outputs of the
+// warps that read it; subnormal numbers are not kept.
+// Measured per application with its launch, FP64 products and these: 64 x 1000 17.3 -> 13.1 us (1.6 TB/s of
+// coefficients, from L2), 65 x 1500 23.0 -> 16.6, 37 x 811 11.1 -> 8.9, 23 x 437 6.4 -> 5.1, 10 x 106 the same.
 constexpr int kFixedBits = 58;
 __global__ void k_band_fixed_slots(const double* __restrict__ slots, int nr, int width, int2* __restrict__ digits,
                                    int* __restrict__ exps) {
@@ -823,7 +831,7 @@ static void band_apply_v(const BandOp<T>& op, const void* x, void* y, const Sche
         band_apply_v<T, KB, 10>(op, x, y, sched, ctrl, scaling, check_broken, s);
         return;
     } else if constexpr (V >= 9) {
-        constexpr int G = V == 9 || V == 11 ? 1 : 2;
+        constexpr int G = V == 9 ? 1 : 2;
         if (sizeof(T) == sizeof(double) || op.slots_lo) {
             const int tw = op.maxt < kTermWarps ? (op.maxt < 1 ? 1 : op.maxt) : kTermWarps;
             dim3 grid((op.nr + 16 * G - 1) / (16 * G), op.nl);
@@ -835,8 +843,8 @@ static void band_apply_v(const BandOp<T>& op, const void* x, void* y, const Sche
         return;
     }
     if constexpr (V >= 6) {
-        // (selected by the host only for complex64 operators with split coefficients and even nr;
-        // vectors not on a 16-byte boundary take the one-element form)
+        // (the host offers them for even nr, for complex64 with split coefficients; complex64 vectors not on a
+        // 16-byte boundary take the one-element form)
         if constexpr (sizeof(T) < sizeof(double)) {
             constexpr int TH = V == 6 ? 128 : V == 7 ? 64 : 32;
             if (op.slots_lo != nullptr && op.nr % 2 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)y & 15) == 0) {

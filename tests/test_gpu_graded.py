@@ -1,0 +1,59 @@
+"""Vectors whose parts differ by many orders: every part keeps its own digits, whatever lies beside it.
+Reference: dense numpy in FP64, on inputs scaled by powers of two where they leave its range."""
+import numpy as np
+import pytest
+
+from pyprop_gb300 import _native
+from test_gpu_band_shapes import _operator
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tuned", [False, True])
+@pytest.mark.parametrize("nl,nr,kb", [(3, 60, 6), (5, 129, 7), (6, 300, 3), (16, 500, 6)])
+@pytest.mark.parametrize("fall", [0.5, 3.0])
+def test_band_elementwise(tuned, nl, nr, kb, fall):
+    """The operator of a handle as it comes and as the autotuner leaves it, on rows that fall by `fall` orders of ten
+    per element towards one end, imaginary parts 1e-20 of the real ones: FP64 rounds each of an element's products
+    and sums once, 2^-53 of its own |A| |x| each (and subnormal results to 2^-1074), numpy the two products of
+    each entry."""
+    import torch
+    rng = np.random.default_rng(nr + kb)
+    h = _native.Handle(nl, nr, _native.FP64, 4, 0, False, 0)
+    h.set_overlap(1, np.tile([0.0, 1.0], nr))
+    ops = _operator(h, rng, nl, nr, kb)
+    h.finalize()
+    if tuned:
+        assert h.autotune() in (9, 10)
+    g = 10.0 ** -np.minimum(fall * np.arange(nr), 300.0)
+    x = rng.standard_normal((nl, nr)) + 1e-20j * rng.standard_normal((nl, nr))
+    x *= np.where(np.arange(nl)[:, None] % 2, g, g[::-1])
+    y = torch.zeros((nl, nr), dtype=torch.complex128, device="cuda")
+    scal = [1.0, 0.37, -1.9]
+    h.matvec(torch.as_tensor(x).cuda(), y, scal[1:], balanced=False)
+    got, want, size, terms = y.cpu().numpy(), np.zeros((nl, nr), complex), np.zeros((2, nl, nr)), np.zeros((nl, 1))
+    for td, rows, cols, M in ops:
+        for r, c, A in zip(rows, cols, M):
+            want[r] += scal[td] * (A @ x[c])
+            a, b = abs(A.real), abs(A.imag)
+            size[0, r] += abs(scal[td]) * (a @ abs(x[c].real) + b @ abs(x[c].imag))
+            size[1, r] += abs(scal[td]) * (a @ abs(x[c].imag) + b @ abs(x[c].real))
+            terms[r] += 2
+    bound = size * 2.0 ** -53 * (3 * (2 * kb + 1) + 4 * terms + 8) + 2.0 ** -1060
+    assert (abs(got.real - want.real) <= bound[0]).all() and (abs(got.imag - want.imag) <= bound[1]).all()
+
+
+def test_band_nonfinite_neighbours():
+    """An infinity reaches the kb elements on either side, as itself, and no other."""
+    import torch
+    nr = 100
+    h = _native.Handle(1, nr, _native.FP64, 4, 0, False, 0)
+    h.set_overlap(1, np.tile([0.0, 1.0], nr))
+    h.add_potential(_native.STORAGE_DIAG, None, 2, np.ones((1, 5 * nr), dtype=np.complex128), False)
+    h.finalize()
+    src = torch.ones((1, nr), dtype=torch.complex128, device="cuda")
+    src[0, 50] = complex(float("inf"), 1.0)
+    dst = torch.zeros_like(src)
+    h.matvec(src, dst, 0.0, balanced=False)
+    re = dst.real[0].cpu().numpy()
+    assert np.isposinf(re[48:53]).all() and (re[3:48] == 5.0).all() and (re[53:97] == 5.0).all()
