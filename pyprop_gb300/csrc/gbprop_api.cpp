@@ -660,7 +660,7 @@ bool set_inv_chunks(gbprop_ctx* h, int batch) {
                 const int chunk = chunk_of(t.n, nch);
                 if (chunk == prev) continue;
                 prev = chunk;
-                for (int lg = 0; lg <= 4 && (lg == 0 || (1 << (lg - 1)) < h->nl); ++lg) {
+                for (int lg = 0; (1 << lg) <= t.warps && (lg == 0 || (1 << (lg - 1)) < h->nl); ++lg) {
                     const double c = solve_cost(h, t, chunk, lg, r64, batch);
                     if (best_cost >= 0.0 && c >= best_cost) continue;
                     if (!set_solve_shape(t, chunk, lg, r64)) break;
@@ -676,7 +676,7 @@ bool set_inv_chunks(gbprop_ctx* h, int batch) {
             h->pinv[dir] = t;
             InvTab one = t;
             best_cost += 6000.0;
-            for (int lg = 0; lg <= 4 && (lg == 0 || (1 << (lg - 1)) < h->nl); ++lg) {
+            for (int lg = 0; (1 << lg) <= t.warps && (lg == 0 || (1 << (lg - 1)) < h->nl); ++lg) {
                 const int chunk = chunk_of(t.n, 1);
                 const double c = solve_cost(h, t, chunk, lg, r64, batch);
                 if (c >= best_cost) continue;
@@ -1511,7 +1511,7 @@ gbprop_status gbprop_autotune(gbprop_handle h, int* variant) {
                 const int chunk = chunk_of(h->nr, nch);
                 if (chunk == prev) continue;
                 prev = chunk;
-                for (int lg = 0; lg <= 4 && (lg == 0 || (1 << (lg - 1)) < h->nl); ++lg)
+                for (int lg = 0; (1 << lg) <= keep.warps && (lg == 0 || (1 << (lg - 1)) < h->nl); ++lg)
                     if (pin_c[dir] > 0 ? chunk == chunk_of(h->nr, pin_c[dir]) : true)
                         cand.push_back({solve_cost(h, keep, chunk, lg, r64, 0), {chunk, lg}});
                 if (chunk <= 16) break;

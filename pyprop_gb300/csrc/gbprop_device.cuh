@@ -106,8 +106,9 @@ __device__ __forceinline__ double2 round_c64(double2 v) {
 //   d2f_fast: round to nearest even, as (float)d for results in FP32's normal range; results
 //             below it are flushed to signed zero; overflow gives +-inf and NaN stays NaN.
 //   f2d_fast: exact, as (double)f, except that subnormal floats become signed zero.
+// With K the float stands for the double times 2^K.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float d2f_fast(double d) {
+template <int K = 0> __device__ __forceinline__ float d2f_fast(double d) {
     const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
     const unsigned sign = hi & 0x80000000u;
     const unsigned e = (hi >> 20) & 0x7ffu;
@@ -115,30 +116,30 @@ __device__ __forceinline__ float d2f_fast(double d) {
     const unsigned rem = lo & 0x1fffffffu;
     const unsigned up = (rem > 0x10000000u) | ((rem == 0x10000000u) & fm & 1u);
     unsigned bits;
-    if (e <= 896u) bits = sign;
-    else if (e >= 1151u) bits = sign | ((e == 2047u && ((hi & 0xfffffu) | lo)) ? 0x7fc00000u : 0x7f800000u);
-    else bits = sign | (((e - 896u) << 23) + fm + up);
+    if (e <= 896u - K) bits = sign;
+    else if (e >= 1151u - K) bits = sign | ((e == 2047u && ((hi & 0xfffffu) | lo)) ? 0x7fc00000u : 0x7f800000u);
+    else bits = sign | (((e - (896u - K)) << 23) + fm + up);
     return __uint_as_float(bits);
 }
 
-// what d2f_fast rounds off, d - (double)d2f_fast(d), to FP32 precision: the 29 mantissa bits below the
+// what d2f_fast rounds off, d 2^K - (double)d2f_fast<K>(d), to FP32 precision: the 29 mantissa bits below the
 // FP32 value as a signed integer, its exponent set by integer addition (zero below FP32's normal range)
-__device__ __forceinline__ float d2f_low(double d) {
+template <int K = 0> __device__ __forceinline__ float d2f_low(double d) {
     const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
     const int e = (int)((hi >> 20) & 0x7ffu);
     const unsigned fm = lo >> 29, rem = lo & 0x1fffffffu;
     const unsigned up = (rem > 0x10000000u) | ((rem == 0x10000000u) & fm & 1u);
     const int r = (int)rem - (up ? 0x20000000 : 0);
     const unsigned f = __float_as_uint((float)r);
-    const int fe = (int)((f >> 23) & 0xffu) + e - 1075;
+    const int fe = (int)((f >> 23) & 0xffu) + e - (1075 - K);
     if (r == 0 || fe <= 0 || fe >= 255) return 0.f;
-    return __uint_as_float((f + ((unsigned)(e - 1075) << 23)) ^ (hi & 0x80000000u));
+    return __uint_as_float((f + ((unsigned)(e - (1075 - K)) << 23)) ^ (hi & 0x80000000u));
 }
 
-__device__ __forceinline__ double f2d_fast(float f) {
+template <int K = 0> __device__ __forceinline__ double f2d_fast(float f) {
     const unsigned u = __float_as_uint(f);
     const unsigned e = (u >> 23) & 0xffu, sign = u & 0x80000000u;
-    const unsigned de = e == 255u ? 2047u : e + 896u;
+    const unsigned de = e == 255u ? 2047u : e + (896u - K);
     const unsigned hi = e == 0 ? sign : (sign | (de << 20) | ((u & 0x7fffffu) >> 3));
     const unsigned lo = e == 0 ? 0u : (u & 0x7u) << 29;
     return __hiloint2double((int)hi, (int)lo);
@@ -147,11 +148,11 @@ __device__ __forceinline__ double f2d_fast(float f) {
 // 2^e as a double, -1022 <= e <= 1023
 __device__ __forceinline__ double pow2_double(int e) { return __hiloint2double((e + 1023) << 20, 0); }
 
-// d * 2^s by the exponent field; zero, subnormals and results below the normal range become signed zero
-__device__ __forceinline__ double scale_pow2(double d, int s) {
-    const int hi = __double2hiint(d), e = ((hi >> 20) & 0x7ff), f = e + s;
-    if (e == 0 || f <= 0) return __hiloint2double(hi & 0x80000000, 0);
-    return __hiloint2double(hi + (s << 20), __double2loint(d));
+// d 2^e, |e| <= 1100: by the exponent field between normal numbers
+__device__ __forceinline__ double scale_pow2(double d, int e) {
+    const int hi = __double2hiint(d), f = (hi >> 20) & 0x7ff;
+    if (f != 0 && f + e > 0 && f + e < 2047 && f != 2047) return __hiloint2double(hi + (e << 20), __double2loint(d));
+    return d == 0.0 ? d : d * pow2_double(e / 2) * pow2_double(e - e / 2);
 }
 
 // ---------------------------------------------------------------------------

@@ -63,7 +63,7 @@ struct InvTab {
     int n, kd, w, npad;
     int ks;                 // k steps of a block
     int lg;                 // log2 of the rows per CTA
-    int warps;              // worker warps per CTA (8 or 16)
+    int warps;              // worker warps per CTA (8 or 16), at least as many as rows
     int chunk, nchunks;
     int refine;             // refinement passes of the FP64-accurate solve
     int stage;

@@ -401,6 +401,9 @@ cudaError_t launch_solve_ir(const void* tabf, const double* udp, int nrows, cons
 // batch, where two or three CTAs of different problems share an SM (InvTab::warps).
 constexpr int kRowWarps = 16;                        // most worker warps
 constexpr int kRowBlock = 32 * kRowWarps + 32;       // + the warp that forms 1/beta
+// The FP64 solve's FP32 and bfloat16 numbers stand for 2^-kBias of themselves (free in the integer conversions): a
+// row of up to 2^50 leaves FP32 room for U^-1 above, one of 2^-100 for its residuals and their parts below
+constexpr int kBias = 40;
 
 __device__ __forceinline__ void worker_sync(int nw) { asm volatile("bar.sync 1, %0;" :: "r"(32 * nw) : "memory"); }
 
@@ -471,6 +474,7 @@ __global__ void __launch_bounds__(kRowBlock) k_solve_rows(InvTab tab, int nl, co
                                                           int scale_mode, int check_broken, const void* bpart, int bG) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned s_red[kRowWarps];
+    __shared__ int s_e[kRowWarps];                     // powers of two of scaled rows (FP64 solve)
     __shared__ double s_ib;                            // 1/beta (FP64 solve)
     __shared__ float2 s_ibf;                           // 1/beta as an FP32 pair (complex64 solve)
     __shared__ int s_brk, s_skip;
@@ -578,8 +582,8 @@ __global__ void __launch_bounds__(kRowBlock) k_solve_rows(InvTab tab, int nl, co
     // right-hand side: a warp takes 32-element segments of the rows, kPre of them loaded at once
     constexpr int kPre = 3;
     const int nbs = ((RB + 31) >> 5) << lg;
-    double fin = 1.0;                                  // R64: factor of x and v at the end, if `scaled`
-    bool scaled = scale_mode != 0;
+    double fin = 1.0;                                  // R64: factor of x and v at the end, if scale_mode
+    bool rescaled = false;                             // R64: rows of b are scaled, row r by 2^-s_e[r]
     if constexpr (R64) {
         if (scale_mode && !late) fin = ctrl->inv_beta;
         auto keep = [&](int it, double2 b) {
@@ -587,11 +591,11 @@ __global__ void __launch_bounds__(kRowBlock) k_solve_rows(InvTab tab, int nl, co
             if (row < rows && q < RB) {
                 bq[row * PB + q] = b;
                 unsigned short* rr = r16 + 2 * row * PQ + q;
-                put_split(rr, PL, d2f_fast(b.x));
-                put_split(rr + PQ, PL, d2f_fast(b.y));
+                put_split(rr, PL, d2f_fast<kBias>(b.x));
+                put_split(rr + PQ, PL, d2f_fast<kBias>(b.y));
             }
         };
-        unsigned hmax = 0;
+        unsigned hmax = 0;                             // (a warp's items are of one row: 2^lg <= nw)
         for (int i0 = warp;;) {
             double2 pre[kPre];
 #pragma unroll
@@ -620,20 +624,29 @@ __global__ void __launch_bounds__(kRowBlock) k_solve_rows(InvTab tab, int nl, co
         if (lane == 0) s_red[warp] = hmax;
         if (STAGE) cp_async_wait_all();
         worker_sync(nw);
-        hmax = __reduce_max_sync(0xffffffffu, s_red[lane & (nw - 1)]);
-        // a right-hand side whose largest exponent leaves the range where the FP32 residuals
-        // (down to 2^-50 of it) stay normal is scaled by a power of two, and x back at the end
-        const int e = (int)(hmax >> 20) - 1022;
-        if (hmax != 0 && hmax < 0x7ff00000u && (e < -60 || e > 60)) {
-            scaled = true;
-            fin = fin * pow2_double(e / 2) * pow2_double(e - e / 2);
-            for (int it = warp; it < nbs; it += nw) {
-                const int row = it & rmask, q = (it >> lg) * 32 + lane;
-                if (row >= rows || q >= RB) continue;
-                const double2 b = bq[row * PB + q];
-                keep(it, make_double2(scale_pow2(b.x, -e), scale_pow2(b.y, -e)));
+        // a row whose largest exponent leaves the range where the FP32 residuals (down to 2^-50 of it) and their
+        // bfloat16 parts stay normal is scaled by a power of two, and its x back at the end.  Every row by its own:
+        // beside a row of magnitude 1 one of 1e-39 would lose everything to FP32's exponent range, and wave functions'
+        // tails are such rows.  s_red[v] is of row v & rmask
+        const unsigned hv = s_red[lane & (nw - 1)];
+        if (__any_sync(0xffffffffu, hv != 0 && hv - ((1022u - 100u) << 20) >= (151u << 20))) {     // outside -100 .. 50
+            unsigned hr = hv;
+            for (int o = 1 << lg; o < nw; o <<= 1) hr = max(hr, __shfl_xor_sync(0xffffffffu, hr, o));
+            const int e = (int)(hr >> 20) - 1022;
+            const int er = hr != 0 && hr < 0x7ff00000u && (e < -100 || e > 50) ? e : 0;      // of row lane & rmask
+            rescaled = __any_sync(0xffffffffu, er != 0);                                    // (the same in every warp)
+            if (rescaled) {
+                if (warp == 0 && lane <= rmask) s_e[lane] = er;
+                const int row = warp & rmask, ew = -__shfl_sync(0xffffffffu, er, row);
+#pragma unroll 1
+                for (int it = warp; it < nbs && ew != 0 && row < rows; it += nw) {
+                    const int q = (it >> lg) * 32 + lane;
+                    if (q >= RB) break;
+                    const double2 b = bq[row * PB + q];
+                    keep(it, make_double2(scale_pow2(b.x, ew), scale_pow2(b.y, ew)));
+                }
+                worker_sync(nw);
             }
-            worker_sync(nw);
         }
     } else {
         if (in_prec == 0) {
@@ -726,7 +739,7 @@ __global__ void __launch_bounds__(kRowBlock) k_solve_rows(InvTab tab, int nl, co
                     float4 b;                          // b's FP32 pairs
                     if constexpr (R64) {
                         const double2 v = bq[row * PB + q];
-                        b = make_float4(d2f_fast(v.x), d2f_fast(v.y), d2f_low(v.x), d2f_low(v.y));
+                        b = make_float4(d2f_fast<kBias>(v.x), d2f_fast<kBias>(v.y), d2f_low<kBias>(v.x), d2f_low<kBias>(v.y));
                     } else {
                         b = bf[row * PB + q];
                     }
@@ -754,8 +767,8 @@ __global__ void __launch_bounds__(kRowBlock) k_solve_rows(InvTab tab, int nl, co
                         r.x = fma(-u, xv.x, r.x);
                         r.y = fma(-u, xv.y, r.y);
                     }
-                    put_split(rr, PL, d2f_fast(r.x));
-                    put_split(rr + PQ, PL, d2f_fast(r.y));
+                    put_split(rr, PL, d2f_fast<kBias>(r.x));
+                    put_split(rr + PQ, PL, d2f_fast<kBias>(r.y));
                 }
             }
             if (R64 && k == P) __syncthreads();        // with the warp that forms 1/beta
@@ -783,14 +796,14 @@ __global__ void __launch_bounds__(kRowBlock) k_solve_rows(InvTab tab, int nl, co
             } else if constexpr (R64) {
                 double2 x[2];
 #pragma unroll
-                for (int j = 0; j < 2; ++j) x[j] = make_double2(f2d_fast(d[2 * j]), f2d_fast(d[2 * j + 1]));
+                for (int j = 0; j < 2; ++j) x[j] = make_double2(f2d_fast<kBias>(d[2 * j]), f2d_fast<kBias>(d[2 * j + 1]));
                 double2* xp = xd + row * PD + q;
                 if (k == 1 && pair) {
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
                         const float2 x0 = x0f[row * PX + q + 8 * j];
-                        x[j].x += f2d_fast(x0.x);
-                        x[j].y += f2d_fast(x0.y);
+                        x[j].x += f2d_fast<kBias>(x0.x);
+                        x[j].y += f2d_fast<kBias>(x0.y);
                     }
                 } else if (k > 0) {
 #pragma unroll
@@ -805,9 +818,14 @@ __global__ void __launch_bounds__(kRowBlock) k_solve_rows(InvTab tab, int nl, co
                     xp[8] = x[1];
                     continue;
                 }
-                if (scaled) {
+                if (scale_mode) {
 #pragma unroll
                     for (int j = 0; j < 2; ++j) x[j] = make_double2(x[j].x * fin, x[j].y * fin);
+                }
+                if (rescaled) {
+                    const int e = s_e[row];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) x[j] = make_double2(scale_pow2(x[j].x, e), scale_pow2(x[j].y, e));
                 }
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
@@ -829,13 +847,16 @@ __global__ void __launch_bounds__(kRowBlock) k_solve_rows(InvTab tab, int nl, co
             }
         }
         if (R64 && last && vstore) {
-            // the basis vector v = in / beta (fin also undoes a power-of-two scaling of b)
+            // the basis vector v = in / beta
+            const int e = rescaled ? s_e[warp & rmask] : 0;
             const int nvs = ((cl + 31) >> 5) << lg;
             for (int it = warp; it < nvs; it += nw) {
                 const int row = it & rmask, q = (it >> lg) * 32 + lane;
                 if (row >= rows || q >= cl) continue;
                 const double2 b = bq[row * PB + q];
-                reinterpret_cast<double2*>(vstore)[gidx(row, q)] = make_double2(b.x * fin, b.y * fin);
+                double2 v = make_double2(b.x * fin, b.y * fin);
+                if (e) v = make_double2(scale_pow2(v.x, e), scale_pow2(v.y, e));
+                reinterpret_cast<double2*>(vstore)[gidx(row, q)] = v;
             }
         }
         if (!last) worker_sync(nw);

@@ -5,6 +5,7 @@ import pytest
 
 from pyprop_gb300 import _native
 from test_gpu_band_shapes import _operator
+from test_gpu_solve_shapes import _dense, _handle, _rhs
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +58,32 @@ def test_band_nonfinite_neighbours():
     h.matvec(src, dst, 0.0, balanced=False)
     re = dst.real[0].cpu().numpy()
     assert np.isposinf(re[48:53]).all() and (re[3:48] == 5.0).all() and (re[53:97] == 5.0).all()
+
+
+# powers of two: the rows of one problem, in turn (the last but one gives subnormal entries)
+ROWS = [0, -100, 0, -130, 3, -127, -60, -61, 61, -400, 900, -1000, -20, -90, -75, -1035, 1]
+
+
+@pytest.mark.parametrize("nl,nr,order", [(2, 40, 7), (9, 200, 7), (16, 129, 7), (17, 64, 4), (33, 300, 7), (64, 437, 9)])
+@pytest.mark.parametrize("in_batch", [False, True])
+@pytest.mark.parametrize("conj", [False, True])
+def test_solve_rows_of_different_magnitude(nl, nr, order, in_batch, conj):
+    """Each row by itself: its residual is summed in FP64, order + 1 terms, and the factor's inverse acts on that.
+    (Subnormal entries are rounded to their spacing.)"""
+    import torch
+    h, U = _handle(nl, nr, order, _native.FP64)
+    batch = _native.Batch([h], autotune=False) if in_batch else None     # (fewer warps per CTA)
+    p = np.array([ROWS[l % len(ROWS)] for l in range(nl)])
+    x = np.ldexp(1.0, p)[:, None] * _rhs(nl, nr, 3 * nl + nr)
+    up = np.ldexp(1.0, -np.maximum(p, -1000))
+    d = torch.as_tensor(x).cuda()
+    y = torch.empty_like(d)
+    h.matvec(d, y, 1.0, balanced=True)
+    h.solve_sqrt_overlap(conj, d)
+    cond = np.linalg.cond(U)
+    tol, spacing = (order + 1) * 2.0 ** -52 * cond, 2.0 ** -1074 * up * np.sqrt(nr)
+    one, both = _dense(U, x * up[:, None], conj), _dense(U, _dense(U, x * up[:, None], False), True)
+    for got, want, t in ((d, one, tol), (y, both, 4 * cond * tol)):
+        err = np.linalg.norm(got.cpu().numpy() * up[:, None] - want, axis=1)
+        assert (err <= t * np.linalg.norm(want, axis=1) + 4 * cond ** 2 * spacing).all()
+    del batch
