@@ -106,7 +106,10 @@ gbprop_status gbprop_add_potential(gbprop_handle h, int storage, int npairs, con
                                    int kb, const double* data, int time_dependent);
 
 /* Build device tables (solve coupling tables, band slots); call once after the
- * overlap and all potentials are set.  Replaces PamPropagator.SetupStep /
+ * overlap and all potentials are set.  Device memory of an FP64 handle: the operator's
+ * bands (8 bytes a coefficient), the Krylov basis (16 bytes an element and vector) and, for
+ * the Gram-Schmidt kernel that multiplies in fixed point, 24 more of those (without memory for
+ * them the FP64 kernel runs).  Replaces PamPropagator.SetupStep /
  * PampWrapper::Setup (PamPropagator.py:29-45, pampwrapper.cpp:74-81). */
 gbprop_status gbprop_finalize(gbprop_handle h);
 

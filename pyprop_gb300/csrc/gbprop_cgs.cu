@@ -364,28 +364,38 @@ __global__ void __launch_bounds__(kFuseThreads) k_arnoldi_cgs(const double2* __r
     }
 }
 
-// The same step with the products in 56-bit fixed point, for chunks of up to kFixedChunk elements whose
+// The same step with the inner products in 56-bit fixed point, for chunks of up to kFixedChunk elements whose
 // basis rows are in shared memory.  A complex product is four FP64 instructions of 64 cycles of a
 // sub-partition, or 12 integer multiply-adds of about 5: every row of V and w is split into two signed
 // 29-bit digits at the largest exponent of the CTA's chunk, and
 //     a x = a1 x1 2^58 + (a1 x0 + a0 x1) 2^29 + a0 x0
 // summed without its last part.  An entry is rounded to 2^-57 of its chunk's largest and a product's
-// dropped part is below 2^-56 of the two chunks' largest, both of either sign; FP64 rounds every partial
-// sum to 2^-53.  A conversion costs what the products of a pair do, so a row is converted once, by the launch that
+// dropped part is below 2^-56 of the two chunks' largest, both of either sign: h errs by that of ||v|| ||w||, where
+// FP64 rounds every partial sum to 2^-53 (measured at 64 x 1000 and 23 x 437: 2^-54 to 2^-56 of ||w||, FP64
+// 2^-53 to 2^-54).  A conversion costs what the products of a pair do, so a row is converted once, by the launch that
 // meets it first, and its digits are kept for the step's later ones (Vd, ev: the step's launches share their
-// chunks).  For w - V h the coefficients are brought to one exponent with their rows'.  w itself stays in
-// FP64, an element or two per thread, and the correction is subtracted in FP64.
+// chunks).
+// w - V h keeps every element's own digits, however small it is beside the others of its chunk: a row whose h_k is
+// within 2^-kSmallRow of the scale of w (the largest h, or ||w|| where it is known) is subtracted in FP64, its real and
+// imaginary part each -- the real parts of the last two or three for a Hermitian operator, whose other h_k are
+// rounding noise -- and the others in FP32, from rows converted with the digits (Vf): 2^-24 of |V_ki h_k| each,
+// together below 2^-53 max|h| |V_ki|, what the h themselves leave open.  (With digits here too half of the elements of a
+// 64 x 1000 step, emulated, err by 2^39 times what FP64 leaves them; so they by 2, and where w is tens of
+// orders below its largest by up to 2^11, from the h_k of rows that hardly overlap with w.)
 // Measured, a launch with its timing events, mean over the 30 vectors of 64 x 1000: FP64 products 27.1 us,
-// digits formed by every launch 22.0, kept 18.4; FP64 pipe 76% -> 3% busy.  At vector 15 the inner products take
-// 6k cycles, the update 6.5k, arriving rows 3k, the barrier 2.5k and the sums over CTAs 3.3k of about 24k.
+// digits formed by every launch 22.0, kept 18.0 (w - V h in digits too, without the small elements' own), this 18.2.
+// At vector 15 the inner products take 6k cycles, arriving rows 3k, the barrier 2.5k and the sums over CTAs 3.3k.
+constexpr int kSmallRow = 36;
+constexpr int kRowBias = 120;                          // Vf holds V 2^120, |V| <= 1: entries down to 2^-246
 constexpr int kFixedOwn = 2;
 constexpr int kFixedChunk = kFixedOwn * kFuseThreads;
 constexpr int kGsBias = 2 * (1075 + 3) - 29;           // exponent of a product of two digits pairs' sums
 
 template <bool DORTH>
-__global__ void __launch_bounds__(kFuseThreads) k_arnoldi_cgs_fixed(const double2* __restrict__ V, long n, int J, int m,
+__global__ void __launch_bounds__(kFuseThreads, 1) k_arnoldi_cgs_fixed(const double2* __restrict__ V, long n, int J, int m,
                                                                     double2* __restrict__ w, double* __restrict__ part,
-                                                                    int4* __restrict__ Vd, int* __restrict__ ev_rows,
+                                                                    int4* __restrict__ Vd, float2* __restrict__ Vf,
+                                                                    int* __restrict__ ev_rows,
                                                                     unsigned* bar, Ctrl* ctrl, double* H, int update,
                                                                     int chunk, double brk_tol) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -394,8 +404,9 @@ __global__ void __launch_bounds__(kFuseThreads) k_arnoldi_cgs_fixed(const double
     __shared__ double red[kFuseThreads / 32];
     __shared__ int2 s_e[kFuseThreads / 32];
     __shared__ int s_ev[kMaxBasis];                    // the rows' exponents
-    __shared__ int4 s_g[kMaxBasis];                    // the column's digits
-    __shared__ int s_eg, s_again;
+    __shared__ float2 s_hf[64];                        // the column's small entries 2^(1023 - s_hx), zero for the others
+    __shared__ unsigned s_big[2][2];                   // rows whose real, imaginary parts are the others
+    __shared__ int s_hx, s_again;
     __shared__ __align__(8) unsigned long long s_bar;
     const int nv = J + 1, G = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long i0 = (long)b * chunk;
@@ -445,10 +456,13 @@ __global__ void __launch_bounds__(kFuseThreads) k_arnoldi_cgs_fixed(const double
         }
     }
     double2 r[kFixedOwn];                              // this thread's elements of w
+    double2 v0[kFixedOwn], v1[kFixedOwn];              // and of the two newest rows
 #pragma unroll
     for (int u = 0; u < kFixedOwn; ++u) {
         const int i = tid + u * kFuseThreads;
         r[u] = i < cl ? ws[i] : make_double2(0.0, 0.0);
+        v0[u] = i < cl ? cache[(size_t)J * chunk + i] : make_double2(0.0, 0.0);
+        v1[u] = i < cl && J > 0 ? V[(size_t)(J - 1) * n + i0 + i] : make_double2(0.0, 0.0);
     }
     double orig2 = 0.0, resid2 = 0.0;                  // warp 0: squared norms before and after a pass
     double pre2 = 0.0;                                 // before the first
@@ -456,14 +470,11 @@ __global__ void __launch_bounds__(kFuseThreads) k_arnoldi_cgs_fixed(const double
     for (;;) {
         // ---- digits of w and, in the first pass, of the newest row -----------------------------
         const bool first = passes == 0;
-        double2 c[kFixedOwn];
         int ew = 0, ev = 0;
 #pragma unroll
         for (int u = 0; u < kFixedOwn; ++u) {
-            const int i = tid + u * kFuseThreads;
-            c[u] = first && i < cl ? cache[(size_t)J * chunk + i] : make_double2(0.0, 0.0);
             ew = max(ew, max(exp_field(r[u].x), exp_field(r[u].y)));
-            ev = max(ev, max(exp_field(c[u].x), exp_field(c[u].y)));
+            ev = max(ev, max(exp_field(v0[u].x), exp_field(v0[u].y)));
         }
         ew = (int)__reduce_max_sync(0xffffffffu, (unsigned)ew);
         ev = (int)__reduce_max_sync(0xffffffffu, (unsigned)ev);
@@ -479,10 +490,11 @@ __global__ void __launch_bounds__(kFuseThreads) k_arnoldi_cgs_fixed(const double
             const int2 x = split29(to_fixed<3>(r[u].x, ew)), y = split29(to_fixed<3>(r[u].y, ew));
             wd[i] = make_int4(x.x, x.y, y.x, y.y);
             if (!first) continue;
-            const int2 p = split29(to_fixed<3>(c[u].x, ev)), q = split29(to_fixed<3>(c[u].y, ev));
+            const int2 p = split29(to_fixed<3>(v0[u].x, ev)), q = split29(to_fixed<3>(v0[u].y, ev));
             const int4 v = make_int4(p.x, p.y, q.x, q.y);
             cd[(size_t)J * chunk + i] = v;
             Vd[(size_t)J * n + i0 + i] = v;
+            Vf[(size_t)J * n + i0 + i] = make_float2(d2f_fast<kRowBias>(v0[u].x), d2f_fast<kRowBias>(v0[u].y));
         }
         if (first && tid == 0) s_ev[J] = ev_rows[J * G + b] = ev;
         __syncthreads();
@@ -544,68 +556,72 @@ __global__ void __launch_bounds__(kFuseThreads) k_arnoldi_cgs_fixed(const double
             for (int k = tid; k < 2 * nv; k += kFuseThreads) ht[k] = passes ? ht[k] + hs[k] : hs[k];
         }
         if (update) {
-            // the column's digits, every h_k 2^(row exponent) at the largest's exponent
+            // which rows are subtracted in FP64, and the others' entries in FP32
             if (warp == 0) {
-                int e[2], ek[2], eg = 0;
-                bool bad = false;
+                int e[2][2], hx = 0;
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        const int k = lane + 32 * u;
+                        e[u][c] = k < nv ? exp_field(hs[2 * k + c]) : 0;
+                        hx = max(hx, e[u][c]);
+                    }
+                hx = (int)__reduce_max_sync(0xffffffffu, (unsigned)hx);
+                if (DORTH) hx = max(hx, (exp_field(passes ? resid2 : pre2) + 1023) / 2);
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     const int k = lane + 32 * u;
-                    const bool on = k < nv;
-                    e[u] = on ? max(exp_field(hs[2 * k]), exp_field(hs[2 * k + 1])) : 0;
-                    const int v = on ? s_ev[k] : 0;
-                    bad |= e[u] == 2047 || v == 2047;
-                    ek[u] = e[u] && v ? e[u] + v : 0;
-                    eg = max(eg, ek[u]);
-                }
-                eg = (int)__reduce_max_sync(0xffffffffu, (unsigned)eg);
-                bad = __any_sync(0xffffffffu, bad);
+                    float g[2] = {0.f, 0.f};
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int k = lane + 32 * u;
-                    if (k >= nv) continue;
-                    const int sh = ek[u] ? min(eg - ek[u], 60) : 60;
-                    auto digits = [&](double h) {
-                        const long long f = to_fixed<3>(h, e[u]);
-                        return split29(sh ? (f + (1ll << (sh - 1))) >> sh : f);
-                    };
-                    const int2 x = digits(hs[2 * k]), y = digits(hs[2 * k + 1]);
-                    s_g[k] = make_int4(x.x, x.y, y.x, y.y);
+                    for (int c = 0; c < 2; ++c) {
+                        const bool big = e[u][c] != 0 && e[u][c] >= hx - kSmallRow;
+                        const unsigned mask = __ballot_sync(0xffffffffu, big);
+                        if (lane == 0) s_big[c][u] = mask;
+                        if (k < nv && !big) g[c] = d2f_fast(scale_pow2(hs[2 * k + c], 1023 - hx));
+                    }
+                    s_hf[k] = make_float2(g[0], g[1]);
                 }
-                if (lane == 0) s_eg = bad ? -1 : eg;
+                if (lane == 0) s_hx = hx;
             }
             __syncthreads();
-            const int eg = s_eg;
+            const int hx = s_hx;
             double nrm = 0.0;
 #pragma unroll
             for (int u = 0; u < kFixedOwn; ++u) {
                 const int i = tid + u * kFuseThreads;
                 if (i >= cl) break;
-                // (at most 2 kMaxBasis products of 2^54, twice as many of 2^55)
-                long long r1 = 0, r0 = 0, i1 = 0, i0s = 0;
-#pragma unroll 4
-                for (int k = 0; k < nv; ++k) {
-                    const int4 v = cd[(size_t)k * chunk + i], g = s_g[k];
-                    const int a = -v.z, c = -v.w;
-                    mad_wide(r1, v.x, g.x);
-                    mad_wide(r0, v.x, g.y);
-                    mad_wide(r0, v.y, g.x);
-                    mad_wide(r1, a, g.z);
-                    mad_wide(r0, a, g.w);
-                    mad_wide(r0, c, g.z);
-                    mad_wide(i1, v.x, g.z);
-                    mad_wide(i0s, v.x, g.w);
-                    mad_wide(i0s, v.y, g.z);
-                    mad_wide(i1, v.z, g.x);
-                    mad_wide(i0s, v.z, g.y);
-                    mad_wide(i0s, v.w, g.x);
+                float sr = 0.f, si = 0.f;
+                const float2* vf = Vf + i0 + i;
+                for (int k0 = 0; k0 < nv; k0 += 8) {          // eight loads in flight, also in the last round
+                    float2 v[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) v[q] = k0 + q < nv ? vf[(size_t)(k0 + q) * n] : make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const float2 g = s_hf[k0 + q];
+                        sr = fmaf(v[q].x, g.x, sr);
+                        sr = fmaf(-v[q].y, g.y, sr);
+                        si = fmaf(v[q].x, g.y, si);
+                        si = fmaf(v[q].y, g.x, si);
+                    }
                 }
-                if (eg < 0) {
-                    r[u] = make_double2(__hiloint2double(0x7ff80000, 0), __hiloint2double(0x7ff80000, 0));
-                } else {
-                    r[u].x -= from_digits(r1, r0, eg - kGsBias);
-                    r[u].y -= from_digits(i1, i0s, eg - kGsBias);
-                }
+                double dr = scale_pow2(f2d_fast<kRowBias>(sr), hx - 1023), di = scale_pow2(f2d_fast<kRowBias>(si), hx - 1023);
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+#pragma unroll 1
+                    for (int q = 0; q < 2; ++q)
+#pragma unroll 1
+                        for (unsigned rows = s_big[c][q]; rows != 0; rows &= rows - 1) {
+                            const int k = 32 * q + __ffs(rows) - 1;
+                            const double2 v = k == J ? v0[u] : k == J - 1 ? v1[u] : V[(size_t)k * n + i0 + i];
+                            const double g = hs[2 * k + c];
+                            dr = fma(c ? -v.y : v.x, g, dr);
+                            di = fma(c ? v.x : v.y, g, di);
+                        }
+                if (hx == 2047) dr = di = __hiloint2double(0x7ff80000, 0);
+                r[u].x -= dr;
+                r[u].y -= di;
                 if (rnd) r[u] = make_double2(f2d_fast(d2f_fast(r[u].x)), f2d_fast(d2f_fast(r[u].y)));
                 if (!DORTH) w[i0 + i] = r[u];
                 nrm = fma(r[u].x, r[u].x, nrm);
@@ -949,7 +965,7 @@ cudaError_t launch_arnoldi_cgs(int prec, const void* V, const void* v0, long n, 
     if (prec == 0) {
         if (Vd && cgs_fixed(cache, chunk))
             return cgs_coop_launch(cgs_kernel_fixed(dorth), grid, smem, s, (const double2*)V, n, J, m, (double2*)w, part, (int4*)Vd,
-                                   ev_rows, bar, ctrl, H, update, chunk, brk_tol);
+                                   (float2*)((int4*)Vd + (size_t)m * n), ev_rows, bar, ctrl, H, update, chunk, brk_tol);
         auto kern = cgs_kernel64(cache, dorth);
         return cgs_coop_launch(kern, grid, smem, s, (const double2*)V, n, J, m, (double2*)w, part, bar, ctrl, H, update,
                                chunk, brk_tol);
@@ -961,7 +977,7 @@ cudaError_t launch_arnoldi_cgs(int prec, const void* V, const void* v0, long n, 
 }
 
 size_t arnoldi_cgs_digits_bytes(int prec, long n, int m, int grid, int cache) {
-    return prec == 0 && cgs_fixed(cache, cgs_chunk(n, grid)) ? (size_t)m * n * sizeof(int4) : 0;
+    return prec == 0 && cgs_fixed(cache, cgs_chunk(n, grid)) ? (size_t)m * n * (sizeof(int4) + sizeof(float2)) : 0;
 }
 
 // resident CTAs per SM of the FP64 form (of both where it may be the fixed-point one)

@@ -273,8 +273,9 @@ cudaError_t launch_arnoldi_finalize(Ctrl* ctrl, double* H, int m, int J, int dou
 cudaError_t launch_arnoldi_cgs(int prec, const void* V, const void* v0, long n, int J, int m, void* w,
                                double* part, unsigned* bar, Ctrl* ctrl, double* H, int update, int grid, int cache,
                                int dorth, double brk_tol, void* Vd, int* ev_rows, cudaStream_t s);
-// FP64, rows cached: the fixed-point form's digits of the step's basis vectors, arnoldi_cgs_digits_bytes bytes at Vd
-// (0: it does not apply), and their chunks' exponents, kMaxBasis * grid at ev_rows.  Null: the FP64 form.
+// FP64, rows cached: the fixed-point form's digits and FP32 values of the step's basis vectors,
+// arnoldi_cgs_digits_bytes bytes at Vd (0: it does not apply), and their chunks' exponents, kMaxBasis * grid at
+// ev_rows.  Null: the FP64 form.
 size_t arnoldi_cgs_digits_bytes(int prec, long n, int m, int grid, int cache);
 // Grid size for the cooperative Gram-Schmidt (0 if it cannot run co-resident).
 int arnoldi_cgs_grid(int prec, long n, int m, int with_v0, int cache, int dorth);

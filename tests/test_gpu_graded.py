@@ -5,6 +5,7 @@ import pytest
 
 from pyprop_gb300 import _native
 from test_gpu_band_shapes import _operator
+from test_gpu_gram_schmidt_shapes import _handle as _diagonal
 from test_gpu_solve_shapes import _dense, _handle, _rhs
 
 pytestmark = pytest.mark.gpu
@@ -87,3 +88,33 @@ def test_solve_rows_of_different_magnitude(nl, nr, order, in_batch, conj):
         err = np.linalg.norm(got.cpu().numpy() * up[:, None] - want, axis=1)
         assert (err <= t * np.linalg.norm(want, axis=1) + 4 * cond ** 2 * spacing).all()
     del batch
+
+
+@pytest.mark.parametrize("nl,nr,m", [(2, 30, 10), (5, 52, 20), (16, 304, 24), (9, 541, 20), (17, 1001, 24), (64, 1500, 18)])
+@pytest.mark.parametrize("dorth", [False, True])
+@pytest.mark.parametrize("small,rows", [(1e-12, False), (1e-30, False), (1e-60, True)])
+def test_step_elementwise(nl, nr, m, dorth, small, rows):
+    """A step of a diagonal operator multiplies every element by its own phase.  Every second element, or every second
+    row, is small; large and small ones take turns on the spectrum, spread evenly over [-1, 1]: every beta is near 1/2
+    and, with m below 2 sqrt(N / 2), the polynomials of the large points are as tame between them, so nothing
+    amplifies roundings: m vectors of at most log2(N) + m roundings of 2^-53 each, for the small elements as for the
+    large.  The step's polynomial is within (1/8)^m / m! of the phase."""
+    import torch
+    rng = np.random.default_rng(nl * nr + m)
+    N = nl * nr
+    weak = (np.arange(N) // (nr if rows else 1)) % 2 == 1
+    line, diag = np.linspace(-1.0, 1.0, N), np.empty(N)
+    order = np.argsort(np.concatenate([np.arange((~weak).sum()) * 2.0 / (~weak).sum(), np.arange(weak.sum()) * 2.0 / weak.sum() + 1e-9]))
+    rank = np.empty(N, dtype=int)
+    rank[order] = np.arange(N)
+    diag[~weak] = rng.permutation(line[rank[:(~weak).sum()]])
+    diag[weak] = rng.permutation(line[rank[(~weak).sum():]])
+    x = rng.standard_normal(N) + 1j * rng.standard_normal(N)
+    x[weak] *= small
+    h = _diagonal(nl, nr, m, dorth, diag)
+    d = torch.as_tensor(x.reshape(nl, nr)).cuda()
+    h.advance(d, np.zeros(1), 0.25)
+    got, want = d.cpu().numpy().ravel(), x * np.exp(-0.25j * diag)
+    for part in (weak, ~weak):
+        err = np.linalg.norm(got[part] - want[part]) / np.linalg.norm(want[part])
+        assert err < m * (np.log2(N) + m) * 2.0 ** -53
