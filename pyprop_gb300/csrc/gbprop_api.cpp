@@ -140,6 +140,11 @@ struct gbprop_ctx {
     InvTab inv[2] = {};               // the Krylov-precision solves: [0]: U^-1, [1]: U^-T
     InvTab sinv[2] = {};              // the FP64-accurate solves of the state (same tables, own chunking)
     InvTab pinv[2] = {};              // those in place: one chunk where that is as fast as a copy
+    // the forms it runs outside batches, kept while it is a member of one (enter_batch, leave_batch)
+    struct {
+        InvTab inv[2], sinv[2], pinv[2];
+        int cgs_grid, cgs_cache, cgs_dgrid, band_variant;
+    } solo = {};
 
     ~gbprop_ctx() {
         if (graph) cudaGraphExecDestroy(graph);
@@ -1456,6 +1461,7 @@ gbprop_status gbprop_autotune(gbprop_handle h, int* variant) {
     if (variant && *variant >= 0) {                  // explicit choice, no timing
         if (!band_variant_available(h, *variant)) return fail(GBPROP_EINVAL, "no such band-kernel variant");
         set_band_variant(h, *variant);
+        h->solo.band_variant = *variant;
         return GBPROP_OK;
     }
     const int kp = h->kprec();
@@ -1912,6 +1918,41 @@ static void batch_forget(gbprop_batch_ctx* b, gbprop_ctx* h) {
 
 namespace {
 
+// A handle takes a batch's forms while it is a member of one and its own again when it leaves the last.
+void enter_batch(gbprop_batch_ctx* b, gbprop_ctx* h) {
+    if (h->batches.empty()) {
+        auto& s = h->solo;
+        for (int dir = 0; dir < 2; ++dir) {
+            s.inv[dir] = h->inv[dir];
+            s.sinv[dir] = h->sinv[dir];
+            s.pinv[dir] = h->pinv[dir];
+        }
+        s.cgs_grid = h->cgs_grid;
+        s.cgs_cache = h->cgs_cache;
+        s.cgs_dgrid = h->cgs_dgrid;
+        s.band_variant = h->band_variant;
+    }
+    h->batches.push_back(b);
+    h->in_batch = true;
+}
+
+void leave_batch(gbprop_batch_ctx* b, gbprop_ctx* h) {
+    h->batches.erase(std::remove(h->batches.begin(), h->batches.end(), b), h->batches.end());
+    if (!h->batches.empty()) return;
+    const auto& s = h->solo;
+    for (int dir = 0; dir < 2; ++dir) {
+        h->inv[dir] = s.inv[dir];
+        h->sinv[dir] = s.sinv[dir];
+        h->pinv[dir] = s.pinv[dir];
+    }
+    h->cgs_grid = s.cgs_grid;
+    h->cgs_cache = s.cgs_cache;
+    h->cgs_dgrid = s.cgs_dgrid;
+    h->expm_max_cluster = 16;
+    h->in_batch = false;
+    set_band_variant(h, s.band_variant);             // (drops the graphs)
+}
+
 // Capture one parallel branch per problem (forked from and joined into the batch stream).
 // what: bit 0 = enter (x = U psi), bit 1 = one step, bit 2 = leave (psi = U^-1 x).
 gbprop_status batch_capture(gbprop_batch b, void* const* psi, int what, cudaGraphExec_t* out, long long* launches) {
@@ -2031,10 +2072,16 @@ gbprop_status gbprop_batch_create(gbprop_batch* out, const gbprop_handle* proble
         grids[p] = arnoldi_cgs_grid_batch(h->kprec(), h->N, h->m, h->d_v0 != nullptr, &caches[p]);
         grid_sum += grids[p];
     }
+    auto give_up = [&](gbprop_status st) {
+        for (gbprop_ctx* h : b->hs)
+            if (std::count(h->batches.begin(), h->batches.end(), b)) leave_batch(b, h);
+        delete b;
+        return st;
+    };
     for (int p = 0; p < count; ++p) {
         gbprop_ctx* h = b->hs[p];
+        enter_batch(b, h);
         h->expm_max_cluster = expm_cluster;
-        h->in_batch = true;
         if (h->inv_ok) set_inv_chunks(h, 1);
         {
             const int sms = grid_reduce_blocks();
@@ -2042,17 +2089,12 @@ gbprop_status gbprop_batch_create(gbprop_batch* out, const gbprop_handle* proble
             const int grid = coop ? grids[p] : 0, cache = caches[p];
             cudaGetLastError();
             if (grid > 0 && !h->d_gridbar) {
-                if (gbprop_status st = h->dalloc(&h->d_gridbar, 64)) {
-                    delete b;
-                    return st;
-                }
+                if (gbprop_status st = h->dalloc(&h->d_gridbar, 64)) return give_up(st);
                 cudaMemsetAsync(h->d_gridbar, 0, 64, h->stream);
             }
             if (grid > 0 && (!h->d_cgs_part || grid > h->cgs_part_grid)) {
-                if (gbprop_status st = h->dalloc(&h->d_cgs_part, arnoldi_cgs_part_doubles(grid) * sizeof(double))) {
-                    delete b;
-                    return st;
-                }
+                if (gbprop_status st = h->dalloc(&h->d_cgs_part, arnoldi_cgs_part_doubles(grid) * sizeof(double)))
+                    return give_up(st);
                 h->cgs_part_grid = grid;
             }
             h->cgs_grid = grid;
@@ -2062,14 +2104,9 @@ gbprop_status gbprop_batch_create(gbprop_batch* out, const gbprop_handle* proble
         }
         drop_graph(h);
         if (autotune) {
-            gbprop_status st = gbprop_autotune(h, nullptr);
-            if (st) {
-                delete b;
-                return st;
-            }
+            if (gbprop_status st = gbprop_autotune(h, nullptr)) return give_up(st);
         }
     }
-    for (gbprop_ctx* h : b->hs) h->batches.push_back(b);
     *out = b;
     return GBPROP_OK;
 }
@@ -2159,13 +2196,8 @@ gbprop_status gbprop_batch_synchronize(gbprop_batch b) {
 gbprop_status gbprop_batch_destroy(gbprop_batch b) {
     if (!b) return GBPROP_OK;
     if (b->stream) cudaStreamSynchronize(b->stream);
-    for (gbprop_handle h : b->hs) {
-        if (!h) continue;
-        h->batches.erase(std::remove(h->batches.begin(), h->batches.end(), b), h->batches.end());
-        h->expm_max_cluster = 16;
-        h->in_batch = false;
-        if (h->inv_ok) set_inv_chunks(h, 0);
-    }
+    for (gbprop_handle h : b->hs)
+        if (h) leave_batch(b, h);
     delete b;
     return GBPROP_OK;
 }

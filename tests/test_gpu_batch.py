@@ -115,3 +115,42 @@ def test_member_destroyed_before_its_batch(destroyed):
     other.advance(psi, np.zeros(1), 0.01)
     other.synchronize()
     assert bool(torch.isfinite(psi.real).all())
+
+
+@pytest.mark.parametrize("precision,dorth", [("fp64", False), ("fp64", True), ("fp32-mixed", False)])
+@pytest.mark.parametrize("autotune", [False, True])
+def test_a_handle_leaves_a_batch_as_it_came(precision, dorth, autotune):
+    """A batch gives its members forms of its own (shapes, grids, kernels, which round differently): alone again a
+    handle takes the same step, bit for bit, as before, and so it does when the first of two batches goes."""
+    import torch
+    from pyprop_gb300 import _native
+    from pyprop_gb300.batch import HydrogenProblem
+    prec = _native.FP64 if precision == "fp64" else _native.FP32_MIXED
+    probs = [HydrogenProblem(lmax=15, nr=300, rmax=100.0, m=16, seed=s) for s in (1, 2)]
+    hs = []
+    for p in probs:
+        hs.append(_native.Handle(p.nl, p.nr, prec, p.m, 0, dorth, 0))
+        hs[-1].set_overlap(p.kd, p.cholesky_band())
+        for storage, pairs, data, td in p.potentials():
+            hs[-1].add_potential(storage, pairs, p.kb, data, td)
+        hs[-1].finalize()
+    h, dt = hs[0], torch.complex128 if precision == "fp64" else torch.complex64
+    x = torch.as_tensor(probs[0].initial_state()).to("cuda", dt)
+
+    def step():
+        y = x.clone()
+        h.advance(y, np.array([0.3, 0.2]), 0.005)
+        h.synchronize()
+        return y.cpu().numpy().tobytes(), h.tuning()
+
+    want = step()
+    for _ in range(2):
+        a = _native.Batch(hs, autotune=autotune)
+        b = _native.Batch(hs[:1], autotune=autotune)
+        a.__del__()
+        b.__del__()
+        assert step() == want
+    assert h.autotune(4) == 4
+    a = _native.Batch(hs, autotune=autotune)
+    a.__del__()
+    assert h.tuning()[0] == 4
