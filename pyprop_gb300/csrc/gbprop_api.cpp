@@ -915,15 +915,20 @@ gbprop_status arm_flags(gbprop_ctx* h) {
     return GBPROP_OK;
 }
 
-gbprop_status report_flags(gbprop_ctx* h, int lu, int nonfinite, int timeout) {
+gbprop_status fail_flags(int lu, int nonfinite, int timeout) {
     if (!lu && !nonfinite && !timeout) return GBPROP_OK;
-    GB_CUDA(cudaMemsetAsync(&h->d_ctrl->lu_info, 0, 3 * sizeof(int), h->stream));
     // the first cause: a wait that gave up leaves stale data behind it; a failed Pade solve
     // leaves the step's exponential undefined, so later norms turn non-finite (the kernels
     // record no LU failure for a Hessenberg matrix that was non-finite already)
     if (timeout) return fail(GBPROP_ETIMEOUT, "a bounded device-side wait gave up (bulk-copy staging or grid barrier)");
     if (lu) return fail(GBPROP_ELU, "Pade denominator singular (LU info " + std::to_string(lu) + ")");
     return fail(GBPROP_ENONFINITE, "non-finite Krylov norm or Hessenberg matrix");
+}
+
+gbprop_status report_flags(gbprop_ctx* h, int lu, int nonfinite, int timeout) {
+    if (!lu && !nonfinite && !timeout) return GBPROP_OK;
+    GB_CUDA(cudaMemsetAsync(&h->d_ctrl->lu_info, 0, 3 * sizeof(int), h->stream));
+    return fail_flags(lu, nonfinite, timeout);
 }
 
 gbprop_status device_errors(gbprop_ctx* h, bool block) {
@@ -2002,15 +2007,11 @@ gbprop_status batch_errors(gbprop_batch b, bool block) {
     b->flags_armed = false;
     const int p = b->h_flags[3] - 1;
     if (p < 0 || p >= (int)b->hs.size()) return GBPROP_OK;
-    gbprop_ctx* h = b->hs[p];
-    if (!h) return GBPROP_OK;
     // clear every member's flags (only members with a failure have any set)
     for (gbprop_ctx* x : b->hs)
         if (x) GB_CUDA(cudaMemsetAsync(&x->d_ctrl->lu_info, 0, 3 * sizeof(int), b->stream));
-    cudaStream_t keep = h->stream;
-    h->stream = b->stream;
-    gbprop_status st = report_flags(h, b->h_flags[0], b->h_flags[1], b->h_flags[2]);
-    h->stream = keep;
+    const gbprop_status st = fail_flags(b->h_flags[0], b->h_flags[1], b->h_flags[2]);
+    if (st == GBPROP_OK) return st;
     set_last_error((std::string(gbprop_last_error()) + " (problem " + std::to_string(p) + " of the batch)").c_str());
     return st;
 }

@@ -154,3 +154,17 @@ def test_a_handle_leaves_a_batch_as_it_came(precision, dorth, autotune):
     a = _native.Batch(hs, autotune=autotune)
     a.__del__()
     assert h.tuning()[0] == 4
+
+
+def test_failure_of_a_destroyed_member_is_reported():
+    """The batch still says that a step went wrong when the problem that failed has been destroyed since."""
+    from pyprop_gb300 import _native
+    from pyprop_gb300.batch import BatchPropagator, HydrogenProblem
+    bp = BatchPropagator([HydrogenProblem(lmax=2, nr=30, rmax=20.0, m=6, seed=s) for s in (1, 2)], autotune=False)
+    bp.psi[1][0, 3] = float("nan")
+    bp.advance(1)
+    bp.handles[1].__del__()
+    with pytest.raises(_native.GbpropError) as e:
+        bp.synchronize()
+    assert "problem 1" in str(e.value) and "non-finite" in str(e.value)
+    bp.synchronize()
