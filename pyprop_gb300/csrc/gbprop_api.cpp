@@ -140,6 +140,7 @@ struct gbprop_ctx {
     InvTab inv[2] = {};               // the Krylov-precision solves: [0]: U^-1, [1]: U^-T
     InvTab sinv[2] = {};              // the FP64-accurate solves of the state (same tables, own chunking)
     InvTab pinv[2] = {};              // those in place: one chunk where that is as fast as a copy
+    bool variant_named = false;       // a caller chose the band variant
     // the forms it runs outside batches, kept while it is a member of one (enter_batch, leave_batch)
     struct {
         InvTab inv[2], sinv[2], pinv[2];
@@ -1467,6 +1468,7 @@ gbprop_status gbprop_autotune(gbprop_handle h, int* variant) {
         if (!band_variant_available(h, *variant)) return fail(GBPROP_EINVAL, "no such band-kernel variant");
         set_band_variant(h, *variant);
         h->solo.band_variant = *variant;
+        h->variant_named = true;
         return GBPROP_OK;
     }
     const int kp = h->kprec();
@@ -1485,6 +1487,7 @@ gbprop_status gbprop_autotune(gbprop_handle h, int* variant) {
     if (const char* env_c = std::getenv("GBPROP_SOLVE_CHUNKS")) std::sscanf(env_c, "%d,%d", &pin_c[0], &pin_c[1]);
     const bool pinned = band_variant_available(h, pin_v);
     if (pinned) best = pin_v;
+    if (!h->in_batch) h->variant_named = pinned;
     // (complex64 members of a batch: the term-per-warp forms are quicker alone but take more of the SMs'
     // issue slots, which the other members want; 24 mixed problems 3.97 ms with them, 3.57 without.  The
     // fixed-point forms are for callers that ask for them: timing must not choose a handle's accuracy)
@@ -2106,6 +2109,9 @@ gbprop_status gbprop_batch_create(gbprop_batch* out, const gbprop_handle* proble
         drop_graph(h);
         if (autotune) {
             if (gbprop_status st = gbprop_autotune(h, nullptr)) return give_up(st);
+        } else if (!h->variant_named && h->kprec() == 1 && h->band_variant >= 9) {
+            // (see gbprop_autotune: not the term-per-warp forms; the quickest or nearly of the others)
+            set_band_variant(h, band_variant_available(h, 7) ? 7 : 4);
         }
     }
     *out = b;

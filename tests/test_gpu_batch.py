@@ -156,6 +156,19 @@ def test_a_handle_leaves_a_batch_as_it_came(precision, dorth, autotune):
     assert h.tuning()[0] == 4
 
 
+def test_complex64_members_leave_the_other_problems_their_issue_slots():
+    """Untuned complex64 members of a batch take none of the term-per-warp forms, unless one was asked for."""
+    from pyprop_gb300 import _native
+    from pyprop_gb300.batch import HydrogenProblem
+    for nr, want in ((60, 7), (61, 4)):
+        hs = [HydrogenProblem(lmax=2, nr=nr, rmax=20.0, m=6, seed=s).handle(_native.FP32_MIXED, 0) for s in (1, 2)]
+        hs[1].autotune(10)
+        b = _native.Batch(hs, autotune=False)
+        assert [h.tuning()[0] for h in hs] == [want, 10]
+        b.__del__()
+        assert [h.tuning()[0] for h in hs] == [9, 10]
+
+
 def test_failure_of_a_destroyed_member_is_reported():
     """The batch still says that a step went wrong when the problem that failed has been destroyed since."""
     from pyprop_gb300 import _native
