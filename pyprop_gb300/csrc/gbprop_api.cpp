@@ -641,16 +641,16 @@ bool set_solve_shape(InvTab& t, int chunk, int lg, int r64) {
     return false;
 }
 
-// Modelled time of that shape, alone on the GPU: SM cycles of the busiest SM, the fixed part shared by
-// up to two resident CTAs.  In a batch: SM cycles of all CTAs (the other problems fill what is free) and,
-// with the weight of the best of 0, 8 and 32 on batches of 4 to 24 problems, those of one, which the
-// problem's chain of kernels waits for.
+// Modelled time of that shape, alone on the GPU: SM cycles of the busiest SM, one CTA after the other (96 registers
+// by 544 threads let one be resident).  In a batch, with 288 threads: SM cycles of all CTAs (the other problems
+// fill what is free) and, with the weight of the best of 0, 8 and 32 on batches of 4 to 24 problems, those of one,
+// which the problem's chain of kernels waits for.
 double solve_cost(const gbprop_ctx* h, const InvTab& t, int chunk, int lg, int r64, int batch) {
     const int sms = grid_reduce_blocks();
     const long ctas = (long)((h->nl + (1 << lg) - 1) >> lg) * ((t.n + chunk - 1) / chunk);
     const double one = solve_cta_cycles(t, chunk, std::min(1 << lg, h->nl), r64, batch ? 8 : 16);
     if (batch) return ctas * (kSolveFixedCycles / 4 + one) + 32 * one;
-    return (double)((ctas + sms - 1) / sms) * one + (double)((ctas + 2 * sms - 1) / (2 * sms)) * kSolveFixedCycles;
+    return (double)((ctas + sms - 1) / sms) * (one + kSolveFixedCycles);
 }
 
 // The model's choice for the Krylov-precision and the state solves; false if nothing fits.
@@ -1514,7 +1514,7 @@ gbprop_status gbprop_autotune(gbprop_handle h, int* variant) {
     // Krylov-precision solve of each direction around the cost model's choice and keep the fastest
     // (batches keep the model's, other problems fill the GPU)
     if (h->inv_ok && !h->in_batch) {
-        // finite non-zero input (0x3f bytes): a zero right-hand side ends the refinement early
+        // finite input of ordinary size (0x3f bytes): zero rows and rows to be rescaled take other paths
         GB_CUDA(cudaMemsetAsync(h->d_s, 0x3f, (size_t)h->N * h->kelem(), s));
         for (int dir = 0; dir < 2; ++dir) {
             const InvTab keep = h->inv[dir];

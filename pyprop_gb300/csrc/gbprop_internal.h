@@ -50,6 +50,8 @@ template <typename T> struct SolveTab {
 // Each CTA owns `chunk` radial elements (a multiple of 16) of `rg` rows and recomputes the halo its
 // refinement passes need; stage = 1 copies the chunk's slices of U~ into shared memory (16-byte
 // asynchronous copies: q0 and npad are multiples of 4).
+// (five k steps are the inverse bands of orders 7 and 8, 52 to 63 columns, in one round of loads; orders 4 to 6, which
+// have three or four, multiply one or two blocks of zeros, order 9 with six a second round of five)
 constexpr int kSolveFrags = 5;
 __host__ __device__ constexpr int inv_upitch(int kd) { return (kd + 1) | 1; }
 
