@@ -586,6 +586,8 @@ __global__ void __launch_bounds__(kFuseThreads, 1) k_arnoldi_cgs_fixed(const dou
             }
             __syncthreads();
             const int hx = s_hx;
+            const unsigned long long big[2] = {s_big[0][0] | (unsigned long long)s_big[0][1] << 32,
+                                               s_big[1][0] | (unsigned long long)s_big[1][1] << 32};
             double nrm = 0.0;
 #pragma unroll
             for (int u = 0; u < kFixedOwn; ++u) {
@@ -607,18 +609,32 @@ __global__ void __launch_bounds__(kFuseThreads, 1) k_arnoldi_cgs_fixed(const dou
                     }
                 }
                 double dr = scale_pow2(f2d_fast<kRowBias>(sr), hx - 1023), di = scale_pow2(f2d_fast<kRowBias>(si), hx - 1023);
+                auto sub = [&](int k, double2 v) {
+                    if (big[0] >> k & 1) {
+                        dr = fma(v.x, hs[2 * k], dr);
+                        di = fma(v.y, hs[2 * k], di);
+                    }
+                    if (big[1] >> k & 1) {
+                        dr = fma(-v.y, hs[2 * k + 1], dr);
+                        di = fma(v.x, hs[2 * k + 1], di);
+                    }
+                };
+                sub(J, v0[u]);
+                if (J > 0) sub(J - 1, v1[u]);
+                // (an operator that is not Hermitian has more of them: four loads in flight)
+                for (unsigned long long rows = (big[0] | big[1]) & ((1ull << max(J - 1, 0)) - 1); rows != 0;) {
+                    int k[4];
+                    double2 v[4];
 #pragma unroll
-                for (int c = 0; c < 2; ++c)
-#pragma unroll 1
-                    for (int q = 0; q < 2; ++q)
-#pragma unroll 1
-                        for (unsigned rows = s_big[c][q]; rows != 0; rows &= rows - 1) {
-                            const int k = 32 * q + __ffs(rows) - 1;
-                            const double2 v = k == J ? v0[u] : k == J - 1 ? v1[u] : V[(size_t)k * n + i0 + i];
-                            const double g = hs[2 * k + c];
-                            dr = fma(c ? -v.y : v.x, g, dr);
-                            di = fma(c ? v.x : v.y, g, di);
-                        }
+                    for (int q = 0; q < 4; ++q) {
+                        k[q] = __ffsll((long long)rows) - 1;      // -1: none left
+                        rows &= rows - 1;
+                        v[q] = k[q] >= 0 ? V[(size_t)k[q] * n + i0 + i] : make_double2(0.0, 0.0);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (k[q] >= 0) sub(k[q], v[q]);
+                }
                 if (hx == 2047) dr = di = __hiloint2double(0x7ff80000, 0);
                 r[u].x -= dr;
                 r[u].y -= di;
