@@ -288,7 +288,8 @@ gbprop_status gbprop_bound_states(int nr, int kd, int nrows, const double* h_ban
  * the radial chunk counts of the two overlap-factor solve directions (U^-1, U^-T; 0 = the
  * block solver).  The environment GBPROP_BAND_VARIANT=v and GBPROP_SOLVE_CHUNKS=n0,n1 make
  * gbprop_autotune use those instead of timing them (a profiler run reproduces a live run's
- * configuration).  No counterpart in the reference. */
+ * configuration; chunks are multiples of 16 elements, so not every count can be had).  No
+ * counterpart in the reference. */
 gbprop_status gbprop_get_tuning(gbprop_handle h, int* band_variant, int* solve_chunks);
 
 /* Batches of independent problems (each a finalized handle, all of one precision,

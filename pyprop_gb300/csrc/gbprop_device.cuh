@@ -333,7 +333,8 @@ __device__ __forceinline__ long long to_fixed(double d, int emax) {
     return hi < 0 ? -v : v;
 }
 
-// the double nearest to f * 2^(emax - 1075 - S); NaN where emax was that of an infinity or a NaN
+// the double nearest to f * 2^(emax - 1075 - S); NaN where emax was that of an infinity or a NaN, zero below the
+// normal range (of sums over unit vectors' entries, which nothing tells from zero)
 template <int S>
 __device__ __forceinline__ double from_fixed(long long f, int emax) {
     const unsigned long long a = f < 0 ? (unsigned long long)-f : (unsigned long long)f;

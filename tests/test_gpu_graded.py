@@ -61,6 +61,41 @@ def test_band_nonfinite_neighbours():
     assert np.isposinf(re[48:53]).all() and (re[3:48] == 5.0).all() and (re[53:97] == 5.0).all()
 
 
+@pytest.mark.parametrize("variant", [11, 12])
+@pytest.mark.parametrize("nl,nr,kb", [(3, 60, 6), (5, 129, 7), (6, 300, 3)])
+def test_fixed_point_window(variant, nl, nr, kb):
+    """The fixed-point band forms, when asked for: an element errs by what its row's largest coefficient and the largest
+    entry that its warp reads (16 or 32 elements and kb on either side) allow, 2^-58 each factor and 2^-60 for the
+    part left out, and the terms' sums by 2^-53; not by what the rest of the row holds."""
+    import torch
+    rng = np.random.default_rng(nr + kb)
+    h = _native.Handle(nl, nr, _native.FP64, 4, 0, False, 0)
+    h.set_overlap(1, np.tile([0.0, 1.0], nr))
+    ops = _operator(h, rng, nl, nr, kb)
+    h.finalize()
+    assert h.autotune(variant) == variant
+    x = rng.standard_normal((nl, nr)) + 1j * rng.standard_normal((nl, nr))
+    g = 10.0 ** (-0.5 * np.arange(nr))
+    x *= np.where(np.arange(nl)[:, None] % 2, g, g[::-1])
+    y = torch.zeros((nl, nr), dtype=torch.complex128, device="cuda")
+    scal = [1.0, 0.37, -1.9]
+    h.matvec(torch.as_tensor(x).cuda(), y, scal[1:], balanced=False)
+    first = np.arange(nr) // (16 * (variant - 10)) * (16 * (variant - 10))
+    ends = [(max(0, t - kb), t + 16 * (variant - 10) + kb) for t in first]
+    big = np.maximum(abs(x.real), abs(x.imag))
+    window = np.array([[row[a:b].max() for a, b in ends] for row in big])
+    want, size, peak, terms = np.zeros((nl, nr), complex), np.zeros((nl, nr)), np.zeros((nl, nr)), np.zeros((nl, 1))
+    for td, rows, cols, M in ops:
+        for r, c, A in zip(rows, cols, M):
+            want[r] += scal[td] * (A @ x[c])
+            size[r] += abs(scal[td]) * ((abs(A.real) + abs(A.imag)) @ (abs(x[c].real) + abs(x[c].imag)))
+            peak[r] += abs(scal[td]) * 2 * (2 * kb + 1) * np.maximum(abs(A.real), abs(A.imag)).max(axis=1) * window[c]
+            terms[r] += 2
+    # (two real products for each of an element's two components)
+    bound = 2 * peak * (2 * 2.0 ** -58 + 2.0 ** -60) + size * 2.0 ** -53 * (2 * (2 * kb + 1) + 4 * terms + 8)
+    assert (abs(y.cpu().numpy() - want) <= bound).all()
+
+
 # powers of two: the rows of one problem, in turn (the last but one gives subnormal entries)
 ROWS = [0, -100, 0, -130, 3, -127, -60, -61, 61, -400, 900, -1000, -20, -90, -75, -1035, 1]
 

@@ -88,6 +88,16 @@ def test_pinned_chunks(monkeypatch, chunks, precision):
     assert _rel(y.cpu().numpy().astype(np.complex128), want) < tol
 
 
+@pytest.mark.parametrize("chunks", [(1, 2), (3, 7), (19, 1)])
+@pytest.mark.parametrize("precision", [_native.FP64, _native.FP32_MIXED])
+def test_pinned_chunks_are_used(monkeypatch, chunks, precision):
+    """(299 elements split into chunks of 304, 160, 112, 48 and 16: multiples of sixteen)"""
+    monkeypatch.setenv("GBPROP_SOLVE_CHUNKS", "%d,%d" % chunks)
+    h, _ = _handle(11, 299, 7, precision)
+    h.autotune()
+    assert tuple(h.tuning()[1]) == chunks
+
+
 @pytest.mark.parametrize("scale", [1e-300, 1e-60, 1e-25, 1e25, 1e60, 1e300])
 def test_fp64_solve_exponent_range(scale):
     import torch
