@@ -41,16 +41,16 @@ FP32_PEAK_TFLOPS = 69.9
 # from one ncu capture of that kernel (capture constants, not measured by this run; the
 # capture each comes from is named in PHASE_TRAFFIC_SOURCE)
 PHASE_TRAFFIC = {
-    ("fp64", "band"): 21564928, ("fp32-mixed", "band"): 20300288,
-    ("fp64", "solve"): 1678336, ("fp32-mixed", "solve"): 826000,
-    ("fp64", "gram_schmidt"): 16450304, ("fp32-mixed", "gram_schmidt"): 8750336,
+    ("fp64", "band"): 20801280, ("fp32-mixed", "band"): 20297472,
+    ("fp64", "solve"): 1680896, ("fp32-mixed", "solve"): 1091584,
+    ("fp64", "gram_schmidt"): 23111936, ("fp32-mixed", "gram_schmidt"): 8238592,
 }
 PHASE_TRAFFIC_SOURCE = {
-    "band": "profiles/band_kernel_hydrogen_large.md (ncu, dram__bytes_read/write.sum, one launch)",
+    "band": "profiles/band_kernel_hydrogen_large.md (ncu --set full, one launch)",
     "solve": "profiles/k_solve_rows_hydrogen_large.md (ncu --set full, one launch; the inverse band and the factor "
              "stay in L2)",
     "gram_schmidt": "profiles/k_arnoldi_cgs_hydrogen_large.md, profiles/k_arnoldi_cgs32_hydrogen_large.md "
-                    "(ncu --set full, Arnoldi step J = 14)",
+                    "(ncu --set full, Arnoldi step J = 13)",
 }
 GOLD_LARGE = os.path.join(ROOT, "tests", "golden", "oracle_large.npz")
 
@@ -142,7 +142,8 @@ def algorithmic_bytes(N, m, s, coef_bytes):
 
 
 def fp64_ops_per_step(N, nr, m, kd, nterms, kb):
-    """Algorithmic FP64 FMA-pipe operations (thread instructions) of one FP64 Krylov step: band
+    """FP64 FMA-pipe operations (thread instructions) of one FP64 Krylov step if every product ran there
+    (the Gram-Schmidt kernel forms its inner products and most of its update from integers and FP32): band
     matvec (2 per real coefficient and complex element, 4 per term factor and element), classical
     Gram-Schmidt (4 per complex product in the dots and in the update, 2 per element of each norm),
     the last refinement residual of the 2m overlap-factor solves (2 per band entry and 2 adds per
@@ -797,20 +798,22 @@ def measure_single(args, precision, device, world, with_e2e=True):
     _, nterms = operator_slots(prob)
     kd = prob.psi.GetRepresentation().radial.kd
     if precision == "fp64":
-        # 2 FMA (4 flops) per real band entry per complex element
+        # 2 FMA (4 flops) per real band entry per complex element (the fixed-point forms multiply integers instead)
         band_flops = nterms * nr * (2 * kd + 1) * 4
         compute = {"unit": "TFLOP/s", "achieved": band_flops / (t_band * 1e-3) / 1e12, "peak": FP64_PEAK_TFLOPS,
-                   "peak_source": "measured FP64 FMA issue rate on GB300", "what": "FP64 FMA"}
+                   "peak_source": "measured FP64 FMA issue rate on GB300",
+                   "what": "FP64 FMA" if prob.Propagator.BandVariant < 11 else "FP64 products as integer multiply-adds"}
     else:
         # error-free products + compensated sums: ~22 FP32 ops per (hi, lo) band entry and component
         band_flops = nterms * nr * (2 * kd + 1) * 2 * 22
         compute = {"unit": "TFLOP/s", "achieved": band_flops / (t_band * 1e-3) / 1e12, "peak": FP32_PEAK_TFLOPS,
                    "peak_source": "measured FP32 FMA issue rate on GB300", "what": "FP32 ops of the compensated sums"}
     compute["frac"] = compute["achieved"] / compute["peak"]
+    band_name = ("k_band_apply" if prob.Propagator.BandVariant < 9 else
+                 "k_band_split" if prob.Propagator.BandVariant < 11 else "k_band_fixed")
     kernels = {"solve": "k_solve_rows (overlap-factor solves U^-1, U^-T)" if precision == "fp64" else
                "k_solve_rows (complex64 basis solves, FP64 state solve)",
-               "band": "k_band_fixed (TensorPotentialMultiply, all terms)" if precision == "fp64" else
-               "k_band_apply (TensorPotentialMultiply, all terms)",
+               "band": band_name + " (TensorPotentialMultiply, all terms)",
                "gram_schmidt": "k_arnoldi_cgs_fixed (cooperative Gram-Schmidt) + k_norm" if precision == "fp64" else
                "k_arnoldi_cgs32 (cooperative Gram-Schmidt) + k_norm",
                "exponential": "k_expm_cluster (Pade scaling-and-squaring)",
@@ -852,7 +855,7 @@ def measure_single(args, precision, device, world, with_e2e=True):
         "gpu_launches": launches,
     }
     if precision == "fp64":
-        # the FP64 step's own bound: FP64 FMA-pipe operations per step against the measured issue rate
+        # all products of an FP64 step against the measured FP64 issue rate
         ops = fp64_ops_per_step(N, nr, m, kd, nterms, kd)
         line["step_fp64_roofline"] = {
             "fp64_ops_per_step": ops, "unit": "TFLOP/s (2 per FMA-pipe operation)",
