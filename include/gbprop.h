@@ -295,8 +295,9 @@ gbprop_status gbprop_get_tuning(gbprop_handle h, int* band_variant, int* solve_c
 /* Batches of independent problems (each a finalized handle, all of one precision,
  * each with its own operator, sizes, Krylov size, time function and time step),
  * advanced together: one step of the batch is a single CUDA graph launch whose
- * branches are the problems' step sequences.  The handles must outlive the batch.
- * autotune != 0 runs gbprop_autotune on every member first. */
+ * branches are the problems' step sequences.  A batch whose handle was destroyed can only be
+ * waited for and destroyed.  autotune != 0 runs gbprop_autotune on every member first.  While a
+ * handle is a member it runs the forms that suit a batch, its own again when it leaves the last. */
 typedef struct gbprop_batch_ctx* gbprop_batch;
 gbprop_status gbprop_batch_create(gbprop_batch* out, const gbprop_handle* problems, int count, int autotune,
                                   void* stream);

@@ -805,14 +805,15 @@ gbprop_status enqueue_arnoldi(gbprop_ctx* h, int dorth, double brk_tol) {
         // classical Gram-Schmidt against v_0..v_J
         if (fused) {
             GB_LAUNCH(launch_arnoldi_cgs(kp, V, h->d_v0s, N, J, m, h->d_r, h->d_cgs_part, h->d_gridbar, h->d_ctrl,
-                                         h->d_H, J < m - 1, h->cgs_grid, h->cgs_cache, 0, brk_tol, h->d_cgs_digits, h->d_cgs_exps, s));
+                                         h->d_H, J < m - 1, h->cgs_grid, h->cgs_cache, 0, brk_tol, h->d_cgs_digits, h->d_cgs_exps,
+                                         h->in_batch, s));
             tick(h, GBPROP_PHASE_GRAM_SCHMIDT);
             continue;
         }
         if (fused_dorth) {
             GB_LAUNCH(launch_arnoldi_cgs(kp, V, nullptr, N, J, m, h->d_r, h->d_cgs_part, h->d_gridbar, h->d_ctrl, h->d_H,
                                          1, h->cgs_dgrid, h->cgs_cache, 1, brk_tol, h->d_cgs_digits,
-                                         h->d_cgs_exps, s));
+                                         h->d_cgs_exps, 0, s));
             tick(h, GBPROP_PHASE_GRAM_SCHMIDT);
             continue;
         }

@@ -391,8 +391,8 @@ constexpr int kFixedOwn = 2;
 constexpr int kFixedChunk = kFixedOwn * kFuseThreads;
 constexpr int kGsBias = 2 * (1075 + 3) - 29;           // exponent of a product of two digits pairs' sums
 
-template <bool DORTH>
-__global__ void __launch_bounds__(kFuseThreads, 1) k_arnoldi_cgs_fixed(const double2* __restrict__ V, long n, int J, int m,
+template <bool DORTH, int PER_SM>
+__global__ void __launch_bounds__(kFuseThreads, PER_SM) k_arnoldi_cgs_fixed(const double2* __restrict__ V, long n, int J, int m,
                                                                     double2* __restrict__ w, double* __restrict__ part,
                                                                     int4* __restrict__ Vd, float2* __restrict__ Vf,
                                                                     int* __restrict__ ev_rows,
@@ -944,8 +944,11 @@ static int cgs_chunk(long n, int grid) { return (int)(((n + grid - 1) / grid + 7
 // but long vectors of small bases).
 static bool cgs_fixed(int cache, int chunk) { return cache && chunk <= kFixedChunk; }
 
-static decltype(&k_arnoldi_cgs_fixed<false>) cgs_kernel_fixed(int dorth) {
-    return dorth ? k_arnoldi_cgs_fixed<true> : k_arnoldi_cgs_fixed<false>;
+// Alone a CTA has its SM to itself and takes 108 registers, 120 with re-orthogonalisation; a batch's members share SMs
+// with each other's CTAs and solves, so theirs stays within 64 (8 words spilled): alone 64 x 1000 18.7 us a vector with
+// the first and 19.5 with the second, 12 uneven problems 7.65 and 7.54 ms.
+static decltype(&k_arnoldi_cgs_fixed<false, 1>) cgs_kernel_fixed(int dorth, int batch) {
+    return dorth ? k_arnoldi_cgs_fixed<true, 1> : batch ? k_arnoldi_cgs_fixed<false, 2> : k_arnoldi_cgs_fixed<false, 1>;
 }
 
 static decltype(&k_arnoldi_cgs<true, false>) cgs_kernel64(int cache, int dorth) {
@@ -974,13 +977,13 @@ static cudaError_t cgs_coop_launch(Kern kern, int grid, size_t smem, cudaStream_
 
 cudaError_t launch_arnoldi_cgs(int prec, const void* V, const void* v0, long n, int J, int m, void* w,
                                double* part, unsigned* bar, Ctrl* ctrl, double* H, int update, int grid, int cache,
-                               int dorth, double brk_tol, void* Vd, int* ev_rows, cudaStream_t s) {
+                               int dorth, double brk_tol, void* Vd, int* ev_rows, int batch, cudaStream_t s) {
     count_launch();
     const int chunk = cgs_chunk(n, grid);
     const size_t smem = arnoldi_cgs_smem(prec, n, J + 1, grid, v0 != nullptr, cache);
     if (prec == 0) {
         if (Vd && cgs_fixed(cache, chunk))
-            return cgs_coop_launch(cgs_kernel_fixed(dorth), grid, smem, s, (const double2*)V, n, J, m, (double2*)w, part, (int4*)Vd,
+            return cgs_coop_launch(cgs_kernel_fixed(dorth, batch), grid, smem, s, (const double2*)V, n, J, m, (double2*)w, part, (int4*)Vd,
                                    (float2*)((int4*)Vd + (size_t)m * n), ev_rows, bar, ctrl, H, update, chunk, brk_tol);
         auto kern = cgs_kernel64(cache, dorth);
         return cgs_coop_launch(kern, grid, smem, s, (const double2*)V, n, J, m, (double2*)w, part, bar, ctrl, H, update,
@@ -997,14 +1000,15 @@ size_t arnoldi_cgs_digits_bytes(int prec, long n, int m, int grid, int cache) {
 }
 
 // resident CTAs per SM of the FP64 form (of both where it may be the fixed-point one)
-static cudaError_t cgs_occupancy64(long n, int grid, int cache, int dorth, size_t smem, int* per_sm) {
+static cudaError_t cgs_occupancy64(long n, int grid, int cache, int dorth, int batch, size_t smem, int* per_sm) {
     auto kern = cgs_kernel64(cache, dorth);
     allow_max_smem(kern);
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, kFuseThreads, smem);
     if (e == cudaSuccess && cgs_fixed(cache, cgs_chunk(n, grid))) {
         int fixed = 0;
-        allow_max_smem(cgs_kernel_fixed(dorth));
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fixed, cgs_kernel_fixed(dorth), kFuseThreads, smem);
+        auto fk = cgs_kernel_fixed(dorth, batch);
+        allow_max_smem(fk);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fixed, fk, kFuseThreads, smem);
         *per_sm = std::min(*per_sm, fixed);
     }
     return e;
@@ -1026,7 +1030,7 @@ int arnoldi_cgs_grid(int prec, long n, int m, int with_v0, int cache, int dorth)
     int per_sm = 0;
     cudaError_t e;
     if (prec == 0) {
-        e = cgs_occupancy64(n, grid, cache, dorth, smem, &per_sm);
+        e = cgs_occupancy64(n, grid, cache, dorth, 0, smem, &per_sm);
     } else {
         auto kern = cache ? k_arnoldi_cgs32<true> : k_arnoldi_cgs32<false>;
         allow_max_smem(kern);
@@ -1058,7 +1062,7 @@ int arnoldi_cgs_grid_batch(int prec, long n, int m, int with_v0, int* cache) {
         int per_sm = 0;
         cudaError_t e;
         if (prec == 0) {
-            e = cgs_occupancy64(n, grid, c, 0, smem, &per_sm);
+            e = cgs_occupancy64(n, grid, c, 0, 1, smem, &per_sm);
         } else {
             auto kern = c ? k_arnoldi_cgs32<true> : k_arnoldi_cgs32<false>;
             allow_max_smem(kern);

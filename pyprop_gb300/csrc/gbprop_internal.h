@@ -271,10 +271,10 @@ cudaError_t launch_arnoldi_finalize(Ctrl* ctrl, double* H, int m, int J, int dou
 // dorth (FP64): re-orthogonalisation passes inside, and the column, the next beta and the breakdown
 // test (brk_tol) complete on return, as launch_arnoldi_finalize leaves them.
 // The complex64 form takes the first vector as FP32 pairs (v0s, see launch_solve_inv) and
-// forms every sum with error-free FP32 transformations.
+// forms every sum with error-free FP32 transformations.  batch: the grid is arnoldi_cgs_grid_batch's.
 cudaError_t launch_arnoldi_cgs(int prec, const void* V, const void* v0, long n, int J, int m, void* w,
                                double* part, unsigned* bar, Ctrl* ctrl, double* H, int update, int grid, int cache,
-                               int dorth, double brk_tol, void* Vd, int* ev_rows, cudaStream_t s);
+                               int dorth, double brk_tol, void* Vd, int* ev_rows, int batch, cudaStream_t s);
 // FP64, rows cached: the fixed-point form's digits and FP32 values of the step's basis vectors,
 // arnoldi_cgs_digits_bytes bytes at Vd (0: it does not apply), and their chunks' exponents, kMaxBasis * grid at
 // ev_rows.  Null: the FP64 form.
