@@ -1959,7 +1959,8 @@ void leave_batch(gbprop_batch_ctx* b, gbprop_ctx* h) {
     h->cgs_dgrid = s.cgs_dgrid;
     h->expm_max_cluster = 16;
     h->in_batch = false;
-    set_band_variant(h, s.band_variant);             // (drops the graphs)
+    cudaStreamSynchronize(h->stream);                // its graphs, dropped next, may be in flight
+    set_band_variant(h, s.band_variant);
 }
 
 // Capture one parallel branch per problem (forked from and joined into the batch stream).
